@@ -115,6 +115,7 @@ struct DColour {
     const T* u1;  // state: black half (already offset by half)
     T* out;       // this colour's half of the other buffer
     const T* f;   // this colour's half of the right-hand side
+    T om;         // the pass's relaxation
     ColourSplit cs;  // interior groups and shell of the vector body (when split)
     int split;       // 1: the vector body's tasks follow cs (interior without boundary code, then the shell)
 };
@@ -264,7 +265,7 @@ __host__ __device__ __forceinline__ bool batch_vector_level(const Lev& L) { retu
 // one group of BATCH_W cells of colour c (thread index t over (P/W) x rows)
 template <class T, class U>
 __device__ __forceinline__ void colour_group_body(const Lev& L, const KOp<T>& op, int c, const U& u,
-                                                  T* __restrict__ out, const T* __restrict__ f, unsigned t)
+                                                  T* __restrict__ out, const T* __restrict__ f, T om, unsigned t)
 {
     constexpr int W = BATCH_W;
     const unsigned ng = (unsigned)L.P / W;
@@ -285,6 +286,7 @@ __device__ __forceinline__ void colour_group_body(const Lev& L, const KOp<T>& op
         const int i = 2 * (h0 + e) + q;
         res.v[e] = i < L.nx ? gs_value(f4.v[e], diag.v[e], off.v[e]) : T(0);
     }
+    relax_group<T, W>(om, u, c, o0, res);
     stv<T, W>(out + o0, res);
 }
 
@@ -294,13 +296,13 @@ __device__ __forceinline__ void batch_colour(const DColour<T>& d, int c, const U
     if (vec && batch_vector_level(d.L)) {
         if (d.split) {
             // the task's block of the split pass (t = block * TPB + thread)
-            if (d.L.uniform) colour_split_block<T, BATCH_W, U, true>(d.L, d.op, c, u, d.out, d.f, d.cs, t / TPB);
-            else colour_split_block<T, BATCH_W, U, false>(d.L, d.op, c, u, d.out, d.f, d.cs, t / TPB);
+            if (d.L.uniform) colour_split_block<T, BATCH_W, U, true>(d.L, d.op, c, u, d.out, d.f, d.cs, d.om, t / TPB);
+            else colour_split_block<T, BATCH_W, U, false>(d.L, d.op, c, u, d.out, d.f, d.cs, d.om, t / TPB);
         } else {
-            colour_group_body<T, U>(d.L, d.op, c, u, d.out, d.f, t);
+            colour_group_body<T, U>(d.L, d.op, c, u, d.out, d.f, d.om, t);
         }
     } else {
-        colour_body<T, KOp<T>, U>(d.L, d.op, c, u, d.out, d.f, t);
+        colour_body<T, KOp<T>, U>(d.L, d.op, c, u, d.out, d.f, d.om, t);
     }
 }
 
@@ -797,7 +799,8 @@ static void plan_batch(BatchState& B, BatchPlan<T>& P, const mps_solver_opts* o,
     auto cur1 = [&](int p, int d) {
         return batch_hier<T>(*B.sub[p]).U[d][bi[p][d]] + B.sub[p]->lev[d].half;
     };
-    auto colour = [&](std::vector<BStep>& list, int d, int c, int zs) {
+    // pre, sw: the pass's place in the V-cycle (its relaxation, pass_omega)
+    auto colour = [&](std::vector<BStep>& list, int d, int c, int zs, bool pre, int sw) {
         step(
             list, B_COLOUR, d, c, zs, [&](int p) { return d < B.sub[p]->nlev - 1; },
             [&](int p) {
@@ -811,6 +814,7 @@ static void plan_batch(BatchState& B, BatchPlan<T>& P, const mps_solver_opts* o,
                 x.u1 = cur1(p, d);
                 x.out = c == 0 ? H.U[d][ri[p][d] ^ 1] : H.U[d][bi[p][d] ^ 1] + L.half;
                 x.f = H.F[d] + (c ? L.half : 0);
+                x.om = (T)pass_omega(sc.relaxed, d, o, pre, sw, c);
                 x.split = batch_vector_level(L) && make_split(L, BATCH_W, x.cs) ? 1 : 0;
                 if (!x.split) std::memset(&x.cs, 0, sizeof(x.cs));
                 if (c == 0) ri[p][d] ^= 1;
@@ -843,8 +847,8 @@ static void plan_batch(BatchState& B, BatchPlan<T>& P, const mps_solver_opts* o,
         for (int d = 0; d < D; d++) {
             const bool z = d > 0 || zero;
             for (int s = 0; s < o->nu1; s++) {
-                colour(list, d, 0, z && s == 0 ? 2 : 0);
-                colour(list, d, 1, z && s == 0 ? 1 : 0);
+                colour(list, d, 0, z && s == 0 ? 2 : 0, true, s);
+                colour(list, d, 1, z && s == 0 ? 1 : 0, true, s);
             }
             step(
                 list, B_RESTRICT, d, 0, 0, [&](int p) { return d < B.sub[p]->nlev - 1; },
@@ -917,8 +921,8 @@ static void plan_batch(BatchState& B, BatchPlan<T>& P, const mps_solver_opts* o,
                     return (MPS_BATCH_PB && o->nu2 >= 1) ? nb(F.half) : nb((long long)F.nx * F.ny * F.nz);
                 });
             for (int s = 0; s < o->nu2; s++) {
-                colour(list, d, 0, 0);
-                colour(list, d, 1, 0);
+                colour(list, d, 0, 0, false, s);
+                colour(list, d, 1, 0, false, s);
             }
         }
     };

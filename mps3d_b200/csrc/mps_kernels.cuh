@@ -57,9 +57,25 @@ struct OtherOnlyU {  // colour c known zero, the other colour read from memory
     __device__ __forceinline__ T ld(const T* p, int off) const { return p ? __ldg(&p[off]) : T(0); }
 };
 
+// the pass's own cells before the pass, for a relaxed pass (relax_to): zero
+// where the accessor's colour is known zero
+template <class T>
+__device__ __forceinline__ T own_at(const ZeroU<T>&, int, long long) { return T(0); }
+template <class T>
+__device__ __forceinline__ T own_at(const OtherOnlyU<T>&, int, long long) { return T(0); }
+template <class T>
+__device__ __forceinline__ T own_at(const CSplit<T>& u, int c, long long o) { return __ldg(&u.half(c)[o]); }
+
+// the Gauss-Seidel value v over-relaxed from the cell's old value: om = 1 is
+// plain Gauss-Seidel (the callers then do not read the old value)
+template <class T>
+__device__ __forceinline__ T relax_to(T om, T v, T own) { return own + om * (v - own); }
+
 // ---------------------------------------------------------------------
 // one colour pass of red-black Gauss-Seidel, out of place:
-//   out[c] = (f[c] - offdiag(u)) / diag, u = state at the start of the pass
+//   out[c] = own + om ((f[c] - offdiag(u)) / diag - own), u = state at the
+// start of the pass, own = its colour-c half; om = 1 unless the level's
+// schedule over-relaxes the pass (pass_omega)
 // (perform_gseidel_smoothing, discretepde.f90:202-229; the reference
 // computes offdiag of all cells before updating a colour, so cells of one
 // colour never see each other's new values -- the same rule holds here at
@@ -67,21 +83,23 @@ struct OtherOnlyU {  // colour c known zero, the other colour read from memory
 // ---------------------------------------------------------------------
 template <class T, class Op, class U>
 __device__ __forceinline__ void colour_body(const Lev& L, const Op& op, int c, const U& u, T* __restrict__ out,
-                                            const T* __restrict__ f, unsigned t)
+                                            const T* __restrict__ f, T om, unsigned t)
 {
     int i, j, k;
     if (!decode(L, t, c, i, j, k)) return;
     T diag, off;
     row_any<T>(op, L, u, i, j, k, diag, off);
-    out[t] = gs_value(__ldg(&f[t]), diag, off);
+    T v = gs_value(__ldg(&f[t]), diag, off);
+    if (om != T(1)) v = relax_to(om, v, own_at(u, c, t));
+    out[t] = v;
 }
 
 template <class T, class Op, class U>
 __global__ void __launch_bounds__(TPB) k_colour(Lev L, Op op, int c, U u, T* __restrict__ out,
-                                                const T* __restrict__ f)
+                                                const T* __restrict__ f, T om)
 {
     pdl_wait();
-    colour_body<T, Op, U>(L, op, c, u, out, f, blockIdx.x * TPB + threadIdx.x);
+    colour_body<T, Op, U>(L, op, c, u, out, f, om, blockIdx.x * TPB + threadIdx.x);
 }
 
 // ---------------------------------------------------------------------
@@ -161,6 +179,22 @@ __device__ __forceinline__ VecW<T, W> zerov()
 #pragma unroll
     for (int e = 0; e < W; e++) r.v[e] = T(0);
     return r;
+}
+
+// own_at for W cells of a row, and the relaxed pass over them
+template <class T, int W>
+__device__ __forceinline__ VecW<T, W> own_group(const ZeroU<T>&, int, int) { return zerov<T, W>(); }
+template <class T, int W>
+__device__ __forceinline__ VecW<T, W> own_group(const OtherOnlyU<T>&, int, int) { return zerov<T, W>(); }
+template <class T, int W>
+__device__ __forceinline__ VecW<T, W> own_group(const CSplit<T>& u, int c, int o0) { return ldv<T, W>(u.half(c) + o0); }
+template <class T, int W, class U>
+__device__ __forceinline__ void relax_group(T om, const U& u, int c, int o0, VecW<T, W>& res)
+{
+    if (om == T(1)) return;
+    const VecW<T, W> own = own_group<T, W>(u, c, o0);
+#pragma unroll
+    for (int e = 0; e < W; e++) res.v[e] = relax_to(om, res.v[e], own.v[e]);
 }
 
 // the row neighbour along y or z of a group (AX = 1 or 2, S = -1/+1): vectors
@@ -434,7 +468,7 @@ struct SmallShape {
 
 template <class T, int W, class U, int MB = ColourShape<T>::MINB>
 __global__ void __launch_bounds__(TPB, MB) k_colourv(Lev L, KOp<T> op, int c, U u, T* __restrict__ out,
-                                                    const T* __restrict__ f, FastDiv divG)
+                                                    const T* __restrict__ f, FastDiv divG, T om)
 {
     pdl_wait();
     GroupIdx G;
@@ -449,6 +483,7 @@ __global__ void __launch_bounds__(TPB, MB) k_colourv(Lev L, KOp<T> op, int c, U 
         const int i = 2 * (G.h0 + e) + G.q;
         res.v[e] = i < L.nx ? gs_value(f4.v[e], diag.v[e], off.v[e]) : T(0);
     }
+    relax_group<T, W>(om, u, c, G.o0, res);
     stv<T, W>(out + G.o0, res);
 }
 
@@ -547,9 +582,9 @@ __global__ void __launch_bounds__(TPB, ResidShape<T>::MINB) k_residv(Lev L, KOp<
 // One thread per coarse cell, natural order.
 // ---------------------------------------------------------------------
 // the coarse level's first red pass from a zero state, written with the
-// restriction: u(red) = f / diag (gs_value with a zero off-diagonal part, as the
-// zero-state colour pass computes it); d holds the coarse rows' diagonals
-// (red half).  u == nullptr: no such write.
+// restriction: u(red) = f / d (gs_value with a zero off-diagonal part, as the
+// zero-state colour pass computes it); d holds the coarse rows' diagonals over
+// the pass's relaxation (red half, k_diag_red).  u == nullptr: no such write.
 template <class T>
 struct RedZ {
     T* u;
@@ -979,7 +1014,7 @@ __global__ void __launch_bounds__(TPB, MB) k_resid_restrict_v(Lev F, Op op, CSpl
 }
 
 // the red pass of a colour pass from a zero state, elementwise: u(red) =
-// f(red) / diag with the red rows' diagonals of k_diag_red (no neighbour is
+// f(red) / d with the red rows' divisors of k_diag_red (no neighbour is
 // read: every one is zero); pads untouched
 template <class T>
 __global__ void __launch_bounds__(TPB) k_red_from_zero(Lev L, const T* __restrict__ f, const T* __restrict__ d,
@@ -992,10 +1027,11 @@ __global__ void __launch_bounds__(TPB) k_red_from_zero(Lev L, const T* __restric
     out[t] = gs_value<T>(f[t], d[t], T(0));
 }
 
-// the diagonal of every red row of a level (the zero-state colour pass's
-// divisor), for the red pass written with the restriction
+// the diagonal of every red row of a level over the first red pass's
+// relaxation om (the zero-state colour pass's divisor), for the red pass
+// written with the restriction
 template <class T, class Op>
-__global__ void __launch_bounds__(TPB) k_diag_red(Lev L, Op op, T* __restrict__ d)
+__global__ void __launch_bounds__(TPB) k_diag_red(Lev L, Op op, T* __restrict__ d, T om)
 {
     pdl_wait();
     const unsigned t = blockIdx.x * TPB + threadIdx.x;
@@ -1003,7 +1039,7 @@ __global__ void __launch_bounds__(TPB) k_diag_red(Lev L, Op op, T* __restrict__ 
     if (!decode(L, t, 0, i, j, k)) return;
     T diag, off;
     row_any<T>(op, L, ZeroU<T>(), i, j, k, diag, off);
-    d[soff(L, i, j, k)] = diag;
+    d[soff(L, i, j, k)] = diag / om;
 }
 
 // coarse ghost rule for the correction (update_boundary_ghostvalues applied
@@ -1380,7 +1416,7 @@ struct ColourSplit {
 template <class T, int W, class U, bool UNI = true>
 __device__ __forceinline__ void colour_split_block(const Lev& L, const KOp<T>& op, int c, const U& u,
                                                    T* __restrict__ out, const T* __restrict__ f,
-                                                   const ColourSplit& cs, unsigned blk)
+                                                   const ColourSplit& cs, T om, unsigned blk)
 {
     int part;
     unsigned idx;
@@ -1402,6 +1438,7 @@ __device__ __forceinline__ void colour_split_block(const Lev& L, const KOp<T>& o
         VecW<T, W> res;
 #pragma unroll
         for (int e = 0; e < W; e++) res.v[e] = gs_value(f4.v[e], diag.v[e], off.v[e]);
+        relax_group<T, W>(om, u, c, o0, res);
         stv<T, W>(out + o0, res);
         return;
     }
@@ -1434,15 +1471,16 @@ __device__ __forceinline__ void colour_split_block(const Lev& L, const KOp<T>& o
         const int i = 2 * (h0 + e) + q;
         res.v[e] = i < L.nx ? gs_value(f4.v[e], diag.v[e], off.v[e]) : T(0);
     }
+    relax_group<T, W>(om, u, c, o0, res);
     stv<T, W>(out + o0, res);
 }
 
 template <class T, int W, class U, int MB, bool UNI = true>
 __global__ void __launch_bounds__(TPB, MB) k_colourv_split(Lev L, KOp<T> op, int c, U u, T* __restrict__ out,
-                                                           const T* __restrict__ f, ColourSplit cs)
+                                                           const T* __restrict__ f, ColourSplit cs, T om)
 {
     pdl_wait();
-    colour_split_block<T, W, U, UNI>(L, op, c, u, out, f, cs, blockIdx.x);
+    colour_split_block<T, W, U, UNI>(L, op, c, u, out, f, cs, om, blockIdx.x);
 }
 
 // ---------------------------------------------------------------------
@@ -1524,13 +1562,14 @@ __global__ void __launch_bounds__(TPB) k_colourv_split_rop(Lev L, ROp<T> op, int
 // r = f - A u stored as R when rout is set, the sums of r^2 and f^2 added to
 // rr and ff
 // ured (when set): the first red pass of a V-cycle from a zero state on the
-// residual as right-hand side, ured = r / diag on the red cells (the diagonal
-// of this operator, rounded to R), which the V-cycle then skips
+// residual as right-hand side, ured = om r / diag on the red cells (the diagonal
+// of this operator, rounded to R; om the pass's relaxation), which the V-cycle
+// then skips
 template <class T, int W, class R, class Op = KOp<T>>
 __device__ __forceinline__ void resid_split_chunk(const Lev& L, const Op& op, const CSplit<T>& u,
                                                   const T* __restrict__ f, R* __restrict__ rout,
                                                   const ColourSplit& cs, unsigned ch, double& rr, double& ff,
-                                                  R* __restrict__ ured = nullptr)
+                                                  R* __restrict__ ured = nullptr, R om = R(1))
 {
     auto group = [&](int j, int k, int g, auto in) {
         constexpr bool IN = decltype(in)::value;
@@ -1561,7 +1600,7 @@ __device__ __forceinline__ void resid_split_chunk(const Lev& L, const Op& op, co
                 const T r = f4.v[e] - (diag.v[e] * u4.v[e] + off.v[e]);
                 const bool ok = IN || 2 * (h0 + e) + q < L.nx;
                 r4.v[e] = ok ? (R)r : R(0);
-                z4.v[e] = ok ? gs_value(r4.v[e], (R)diag.v[e], R(0)) : R(0);
+                z4.v[e] = ok ? om * gs_value(r4.v[e], (R)diag.v[e], R(0)) : R(0);
                 if (ok) {
                     rr += (double)r * (double)r;
                     ff += (double)f4.v[e] * (double)f4.v[e];
@@ -1605,7 +1644,8 @@ template <class T, int W, class R, class Op = KOp<T>>
 __global__ void __launch_bounds__(TPB, ResidShape<T>::MINB) k_residv_split(Lev L, Op op, CSplit<T> u,
                                                                            const T* __restrict__ f,
                                                                            R* __restrict__ rout, RedBuf rb,
-                                                                           ColourSplit cs, R* __restrict__ ured)
+                                                                           ColourSplit cs, R* __restrict__ ured,
+                                                                           R om)
 {
     pdl_wait();
     __shared__ double sh[32];
@@ -1613,7 +1653,7 @@ __global__ void __launch_bounds__(TPB, ResidShape<T>::MINB) k_residv_split(Lev L
     // block-sized chunks, grid-stride, in the interleaved order of split_chunk
     const unsigned nchunks = cs.nb_in + cs.nb_xe + cs.nb_face;
     for (unsigned ch = blockIdx.x; ch < nchunks; ch += gridDim.x)
-        resid_split_chunk<T, W, R, Op>(L, op, u, f, rout, cs, ch, rr, ff, ured);
+        resid_split_chunk<T, W, R, Op>(L, op, u, f, rout, cs, ch, rr, ff, ured, om);
     const double a = block_sum(rr, sh);
     const double b = block_sum(ff, sh);
     if (!rb.partial) return;
@@ -1884,6 +1924,8 @@ __global__ void k_find_bvec(Lev L, const double* __restrict__ vel, const double*
 // aggregation average (volume weighted for the geometric hierarchy) of a
 // split FP64 field onto the next coarser level
 __global__ void k_restrict_field(Lev F, CSplit<double> in, Lev C, Split<double> out, int geom);
+__global__ void k_restrict_coef(Lev F, CSplit<double> in, CSplit<double> ina, Lev C, Split<double> out,
+                                Split<double> outa);
 
 // rows of the upwind (find_AX) or Scharfetter-Gummel operator from split FP64
 // cell fields of one level

@@ -87,6 +87,7 @@ template <class T>
 struct SubPlan {
     int nl;                   // levels; geo[nl-1] is the coarsest
     int nu1, nu2;             // pre/post red-black sweeps
+    T om0, om1;               // relaxation of the first pre-smoothing sweep and of the later passes (sub_omega)
     int only_black;           // the prolongation corrects the black cells only (nu2 >= 1)
     int gsz;                  // lanes per row of the coarsest solve (power of two, <= 32)
     int nlin, nax, nrow;      // prolongation brackets / axis entries / rows
@@ -148,10 +149,21 @@ __device__ __forceinline__ int sub_gidx(const SubGeo<T>& G, int i, int j, int k)
     return (i + 1) + G.gx * ((j + 1) + G.gy * (k + 1));
 }
 
-// one red-black colour pass of level s, in place.  Thread t takes the cells
-// h = t mod nh of the rows t / nh, t / nh + rc, ...
+// the relaxation of one pass (the per-level launches' pass_omega): the last
+// black pass before the restriction stays plain (the restriction counts on its
+// vanishing residual) and so does the first red pass after the prolongation
+// (which corrects the black cells only)
+template <class T>
+__device__ __forceinline__ T sub_omega(const SubPlan<T>& P, int pre, int sw, int c)
+{
+    if (pre) return c == 1 && sw == P.nu1 - 1 ? T(1) : (sw == 0 ? P.om0 : P.om1);
+    return c == 0 && sw == 0 ? T(1) : P.om1;
+}
+
+// one red-black colour pass of level s, in place, relaxed by om.  Thread t
+// takes the cells h = t mod nh of the rows t / nh, t / nh + rc, ...
 template <class T, bool KF, bool DF>
-__device__ __forceinline__ void sub_colour(const SubPlan<T>& P, const SubMem<T>& M, int s, int c)
+__device__ __forceinline__ void sub_colour(const SubPlan<T>& P, const SubMem<T>& M, int s, int c, T om)
 {
     const SubGeo<T>& G = P.geo[s];
     const int nx = G.nx, ny = G.ny, nh = G.nh, rows = G.rows, rc = G.rc, ax0 = G.ax0;
@@ -173,7 +185,8 @@ __device__ __forceinline__ void sub_colour(const SubPlan<T>& P, const SubMem<T>&
             T ds, as;
             sub_faces<T, KF>(M.ax, ax0, nx, ny, u, kg, kc, i, R.j, R.k, g, ds, as);
             const T d = (DF ? df[idx] : dexc) + T(0.5) * ds;
-            u[g] = gs_value<T>(f[idx], d, T(-0.5) * as);
+            const T v = gs_value<T>(f[idx], d, T(-0.5) * as);
+            u[g] = om != T(1) ? relax_to(om, v, u[g]) : v;
         }
     }
     __syncthreads();
@@ -491,8 +504,8 @@ __global__ void __launch_bounds__(SUB_TPB, 1) k_subcycle(const __grid_constant__
     __syncthreads();
     for (int s = 0; s < P.nl - 1; s++) {
         for (int sw = 0; sw < P.nu1; sw++) {
-            sub_colour<T, KF, DF>(P, M, s, 0);
-            sub_colour<T, KF, DF>(P, M, s, 1);
+            sub_colour<T, KF, DF>(P, M, s, 0, sub_omega(P, 1, sw, 0));
+            sub_colour<T, KF, DF>(P, M, s, 1, sub_omega(P, 1, sw, 1));
         }
         sub_restrict<T, KF, DF>(P, M, s);
     }
@@ -500,8 +513,8 @@ __global__ void __launch_bounds__(SUB_TPB, 1) k_subcycle(const __grid_constant__
     for (int s = P.nl - 2; s >= 0; s--) {
         sub_prolong<T>(P, M, s);
         for (int sw = 0; sw < P.nu2; sw++) {
-            sub_colour<T, KF, DF>(P, M, s, 0);
-            sub_colour<T, KF, DF>(P, M, s, 1);
+            sub_colour<T, KF, DF>(P, M, s, 0, sub_omega(P, 0, sw, 0));
+            sub_colour<T, KF, DF>(P, M, s, 1, sub_omega(P, 0, sw, 1));
         }
     }
     {

@@ -203,7 +203,7 @@ __host__ __device__ inline size_t tma_smem_bytes(const TmaColour& tc)
 
 template <class T, int W, int TJ, bool KF, bool UNI = true>
 __global__ void __launch_bounds__(TJ * 32) k_colour_tma(Lev L, KOp<T> op, int c, CSplit<T> u, T* __restrict__ out,
-                                                        const T* __restrict__ f, ColourSplit cs, TmaColour tc,
+                                                        const T* __restrict__ f, ColourSplit cs, TmaColour tc, T om,
                                                         const __grid_constant__ CUtensorMap tmU,
                                                         const __grid_constant__ CUtensorMap tmKo,
                                                         const __grid_constant__ CUtensorMap tmKc,
@@ -243,6 +243,7 @@ __global__ void __launch_bounds__(TJ * 32) k_colour_tma(Lev L, KOp<T> op, int c,
                 const int i = 2 * (h0 + e) + q;
                 res.v[e] = i < L.nx ? gs_value(f4.v[e], diag.v[e], off.v[e]) : T(0);
             }
+            relax_group<T, W>(om, u, c, o0, res);
             stv<T, W>(out + o0, res);
         }
         return;
@@ -312,16 +313,22 @@ __global__ void __launch_bounds__(TJ * 32) k_colour_tma(Lev L, KOp<T> op, int c,
             const T* Kc = KF ? slotKc(k) + w * P : nullptr;
             const T* Fr = slotF(k) + w * P;
             const int q = (j + k + c) & 1;
-            T* orow = out + (size_t)P * (j + (size_t)L.ny * k);
+            const size_t ro = (size_t)P * (j + (size_t)L.ny * k);
+            T* orow = out + ro;
+            const T* urow = u.half(c) + ro;  // the cells' old values (relaxed passes only)
             for (int g = tc.g_lo + lane; g <= tc.g_hi; g += 32) {
                 const int h0 = W * g;
                 VecW<T, W> diag, off;
+                const VecW<T, W> own = om != T(1) ? ldv<T, W>(urow + h0) : zerov<T, W>();
                 tile_rows<T, W, KF>(op, U0, Uym, Uyp, Uzm, Uzp, K0, Kym, Kyp, Kzm, Kzp, Kc, h0, q, cr0, cr1, cr2, diag,
                                     off);
                 const VecW<T, W> f4 = lds<T, W>(Fr + h0);
                 VecW<T, W> res;
 #pragma unroll
-                for (int e = 0; e < W; e++) res.v[e] = gs_value(f4.v[e], diag.v[e], off.v[e]);
+                for (int e = 0; e < W; e++) {
+                    res.v[e] = gs_value(f4.v[e], diag.v[e], off.v[e]);
+                    if (om != T(1)) res.v[e] = relax_to(om, res.v[e], own.v[e]);
+                }
                 stv<T, W>(orow + h0, res);
             }
         }
