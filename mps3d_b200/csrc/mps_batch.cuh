@@ -623,6 +623,7 @@ static int sub_init(Ctx& parent, Ctx& sc)
     sc.dev = parent.dev;
     sc.nsm = parent.nsm;
     sc.s = parent.s;
+    sc.sub_allowed = false;  // the batched steps run every level themselves
     if (cudaEventCreate(&sc.e0) != cudaSuccess || cudaEventCreate(&sc.e1) != cudaSuccess ||
         cudaMallocHost((void**)&sc.hpin, sizeof(double) * 512) != cudaSuccess ||
         cudaMalloc((void**)&sc.dmax, sizeof(unsigned long long) * 8) != cudaSuccess)

@@ -51,7 +51,7 @@ static_assert(offsetof(mps_problem, timederiv) == 40 && offsetof(mps_problem, dt
               "mps_problem layout");
 #include "mps_kernels.cuh"
 #include "mps_tma.cuh"
-#include "mps_subcycle.cuh"
+#include "mps_cluster.cuh"
 
 #include <cudaTypedefs.h>
 
@@ -156,9 +156,9 @@ struct Hier {
     KOp<T> kop[MAXL];
     ROp<T> rop[MAXL];
     double* AinvT = nullptr;
-    unsigned char* subimg = nullptr;  // solve-constant image of the one-block sub-cycle (k_sub_image)
-    size_t subimg_bytes = 0;
-    bool sub_ok = false;              // the image is current: the V-cycle may run k_subcycle
+    int cl_l0 = -1;                   // first level of the cluster's V-cycle (k_cluster), -1: none
+    unsigned char* cltab = nullptr;   // its axis and interpolation tables
+    T* crow[MAXL] = {};               // explicit rows of a cell coefficient on its levels (k_krows)
     double* Dprev = nullptr;  // the coarsest matrix whose inverse AinvT holds
     int* gj = nullptr;        // its inversion state (k_gauss_jordan)
 };
@@ -236,7 +236,6 @@ struct Ctx {
     bool redz[MAXL] = {};     // level l's first red pass from zero was written by the restriction into it
     bool sub_allowed = true;  // MPS_SUBCYCLE=0 at handle creation: one launch per pass on every level (for comparisons)
     bool relaxed = false;     // over-relaxed passes and averaged-face coarse coefficients (solve_impl)
-    int sub_l0 = -1;          // first level of the one-block sub-cycle (k_subcycle), -1: none
     size_t inbuf_bytes = 0;
     Signature sig;
     int nlev = 0;
@@ -1051,276 +1050,312 @@ static int coarse_solve(Ctx& ctx, Hier<T>& H, int l)
     return 0;
 }
 
-// ---- the small levels in one block (k_subcycle) ----
-// the shared-memory limit of the sub-cycle kernels, set outside any stream
-// capture (at workspace set-up)
-static bool sub_prepare(int dev)
+// ---- the small levels in one cluster (k_cluster) ----
+// the kernel's attributes, set outside any stream capture (at workspace
+// set-up); false when the device cannot hold a cluster of 16 blocks
+static bool cl_prepare(int dev)
 {
     static signed char state[64] = {};
     return once_per_device(dev, state, [] {
         auto set = [](const void* kern) {
-            return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SUB_SMEM_MAX) == cudaSuccess;
+            if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, CL_SMEM_MAX) != cudaSuccess ||
+                cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
+                return false;
+            cudaLaunchConfig_t cfg;
+            std::memset(&cfg, 0, sizeof(cfg));
+            cfg.gridDim = dim3(CL_MAXC);
+            cfg.blockDim = dim3(CL_TPB);
+            cfg.dynamicSmemBytes = CL_SMEM_MAX;
+            cudaLaunchAttribute at[1];
+            at[0].id = cudaLaunchAttributeClusterDimension;
+            at[0].val.clusterDim.x = CL_MAXC;
+            at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+            cfg.attrs = at;
+            cfg.numAttrs = 1;
+            int n = 0;
+            return cudaOccupancyMaxActiveClusters(&n, kern, &cfg) == cudaSuccess && n >= 1;
         };
-        const bool ok = set((const void*)k_subcycle<float, false, false>) && set((const void*)k_subcycle<float, true, false>) &&
-                        set((const void*)k_subcycle<float, false, true>) && set((const void*)k_subcycle<float, true, true>) &&
-                        set((const void*)k_subcycle<double, false, false>) && set((const void*)k_subcycle<double, true, false>) &&
-                        set((const void*)k_subcycle<double, false, true>) && set((const void*)k_subcycle<double, true, true>);
+        const bool ok = set((const void*)k_cluster<float, false>) &&
+                        set((const void*)k_cluster<float, true>) &&
+                        set((const void*)k_cluster<double, false>) &&
+                        set((const void*)k_cluster<double, true>);
         if (!ok) cudaGetLastError();
         return ok;
     });
 }
 
-// first level of the one-block sub-cycle, or -1: the geometric hierarchy, a
-// level below the finest with at most SUB_MAX_CELLS cells and at most
-// SUB_MAXL levels from it to the coarsest (two at least), and no odd periodic
-// size on those levels (cells of one colour would touch, and in-place passes
-// would read new values)
-static int sub_first_level(const Ctx& ctx, const mps_solver_opts* o)
-{
-    if (o->hierarchy != MPS_HIER_GEOM) return -1;
-    const int nl = ctx.nlev;
-    int l0 = -1;
-    for (int l = 1; l < nl - 1; l++) {
-        const Lev& L = ctx.lev[l];
-        if ((long long)L.nx * L.ny * L.nz <= SUB_MAX_CELLS && nl - l <= SUB_MAXL) { l0 = l; break; }
-    }
-    if (l0 < 0) return -1;
-    for (int l = l0; l < nl; l++) {
-        if (odd_periodic(ctx.lev[l])) return -1;
-        if (l < nl - 1 && !ctx.xf[l].geom) return -1;
-    }
-    return l0;
-}
-
-// the ghosted row pitch of a level in the block: nx+2, or 24 for FP32 rows of
-// 16 cells (8 per colour), so that the four rows a warp takes in a colour pass
-// (stride-2 accesses) fall on distinct banks
+// the axis entries of one level in the ghosted layout of row pitch gx: the
+// face coefficients of fcoef / dcoef by position
 template <class T>
-static int sub_gx(const Lev& L)
-{
-    return (sizeof(T) == 4 && L.nh == 8 && L.nx + 2 <= 24) ? 24 : L.nx + 2;
-}
-
-// one level of the block's plan: Lev's sizes, widths and boundary flags
-template <class T>
-static SubGeo<T> sub_geo(const Lev& L)
-{
-    SubGeo<T> G;
-    std::memset(&G, 0, sizeof(G));
-    G.nx = L.nx; G.ny = L.ny; G.nz = L.nz; G.nh = L.nh;
-    G.rows = L.ny * L.nz;
-    G.rc = SUB_TPB / L.nh;
-    G.rn = SUB_TPB / L.nx;
-    G.gx = sub_gx<T>(L);
-    G.gy = L.ny + 2;
-    G.pitch = L.P;
-    for (int a = 0; a < 3; a++) {
-        G.per |= L.per[a] ? 1 << a : 0;
-        G.w[a] = (T)L.w[a];
-        G.wl[a] = (T)L.wl[a];
-    }
-    for (int f = 0; f < 6; f++) G.dirc |= L.bc[f] == BC_DIRC && !L.per[f / 2] ? 1 << f : 0;
-    G.dnh.init((unsigned)L.nh);
-    G.dny.init((unsigned)L.ny);
-    G.dnx.init((unsigned)L.nx);
-    return G;
-}
-
-// the axis entries of one level (ghosted strides 1, nx+2, (nx+2)(ny+2)): the
-// face coefficients of fcoef / dcoef by position, periodic faces wrapping
-template <class T>
-static void sub_axes(const Lev& L, SubAx<T>* out)
+static void cl_axes(const Lev& L, int gx, std::vector<ClAx<T>>& out)
 {
     const int n3[3] = {L.nx, L.ny, L.nz};
-    const int gx = sub_gx<T>(L);
     const int st3[3] = {1, gx, gx * (L.ny + 2)};
-    int e = 0;
     for (int a = 0; a < 3; a++) {
         const int n = n3[a], st = st3[a];
-        const bool per = L.per[a] != 0;
+        const bool per = L.per[a] != 0, wrap = per && a < 2;  // along z the ghost planes hold the wrapped cells
         const bool dm = !per && L.bc[2 * a] == BC_DIRC, dp = !per && L.bc[2 * a + 1] == BC_DIRC;
-        for (int p = 0; p < n; p++, e++) {
-            SubAx<T> x;
-            if (p > 0) { x.om = -st; x.cm = (T)(p == n - 1 ? L.cl[a] : L.cr[a]); }
-            else if (per) { x.om = (n - 1) * st; x.cm = (T)(n == 1 ? L.cl[a] : L.cp[a]); }
-            else { x.om = -st; x.cm = dm ? (T)(n == 1 ? L.dlast[a] : L.dr[a]) : T(0); }
-            if (p < n - 1) { x.op = st; x.cp = (T)(p + 1 == n - 1 ? L.cp[a] : L.cr[a]); }
-            else if (per) { x.op = -(n - 1) * st; x.cp = (T)L.cl[a]; }
-            else { x.op = st; x.cp = dp ? (T)L.dlast[a] : T(0); }
-            out[e] = x;
+        for (int p = 0; p < n; p++) {
+            ClAx<T> x;
+            x.om = -st;
+            x.op = st;
+            if (p > 0) x.cm = (T)(p == n - 1 ? L.cl[a] : L.cr[a]);
+            else if (per) x.cm = (T)(n == 1 ? L.cl[a] : L.cp[a]);
+            else x.cm = dm ? (T)(n == 1 ? L.dlast[a] : L.dr[a]) : T(0);
+            if (p < n - 1) x.cp = (T)(p + 1 == n - 1 ? L.cp[a] : L.cr[a]);
+            else if (per) x.cp = (T)L.cl[a];
+            else x.cp = dp ? (T)L.dlast[a] : T(0);
+            if (wrap && p == 0) x.om = (n - 1) * st;
+            if (wrap && p == n - 1) x.op = -(n - 1) * st;
+            out.push_back(x);
         }
     }
 }
 
-// the block's plan from level l0 for word type T: shared-memory layout
-// (dynamic fields, the solve-constant image, tables), per-level geometry,
-// axis entries and prolongation brackets.  false when it does not fit.
+// the launch plan from level l0: split levels and their planes, shared-memory
+// layout, tables (ax, lin); false when it does not fit
 template <class T>
-static bool sub_layout_with(const Ctx& ctx, int l0, bool kf, bool df, const mps_solver_opts* o, SubPlan<T>& P,
-                            size_t& smem, bool ainv_in_smem);
-
-// the layout with the coarsest inverse staged in shared memory when that fits,
-// else read from device memory by the coarsest solve
-template <class T>
-static bool sub_layout(const Ctx& ctx, int l0, bool kf, bool df, const mps_solver_opts* o, SubPlan<T>& P,
-                       size_t& smem)
-{
-    return sub_layout_with<T>(ctx, l0, kf, df, o, P, smem, true) ||
-           sub_layout_with<T>(ctx, l0, kf, df, o, P, smem, false);
-}
-
-template <class T>
-static bool sub_layout_with(const Ctx& ctx, int l0, bool kf, bool df, const mps_solver_opts* o, SubPlan<T>& P,
-                            size_t& smem, bool ainv_in_smem)
+static bool cl_layout(const Ctx& ctx, int l0, bool rows, ClPlan<T>& P, size_t& smem, std::vector<ClAx<T>>& ax,
+                      std::vector<ClLin<T>>& lin)
 {
     std::memset(&P, 0, sizeof(P));
-    if (l0 < 1 || ctx.nlev - l0 < 2) return false;
+    ax.clear();
+    lin.clear();
     const int nl = ctx.nlev - l0;
+    if (nl < 2 || nl > CL_MAXL) return false;
     P.nl = nl;
-    P.nu1 = o->nu1;
-    P.nu2 = o->nu2;
-    P.om0 = (T)(ctx.relaxed ? OMEGA_FIRST : 1.0);
-    P.om1 = (T)(ctx.relaxed ? OMEGA_LATER : 1.0);
-    P.only_black = o->nu2 >= 1;
-    int nax = 0, nrow = 0, nlin = 0;
-    long long off = 0;  // elements of T: u (ghosted) and f of every level
+    P.geom = ctx.xf[l0].geom;
+    auto cells = [&](int s) { const Lev& L = ctx.lev[l0 + s]; return (long long)L.nx * L.ny * L.nz; };
+    P.m = 0;
+    while (P.m < nl - 1 && cells(P.m) > CL_GATHER) P.m++;
+    P.nc = 1;
+    if (P.m > 0) {
+        // the planes of the coarsest split level over the blocks; a finer plane
+        // belongs to the block of its parent
+        const int nzb = ctx.lev[l0 + P.m - 1].nz;
+        P.nc = std::min(CL_MAXC, nzb);
+        for (int s = P.m - 1; s >= 0; s--) {
+            ClLev<T>& G = P.lev[s];
+            const int nz = ctx.lev[l0 + s].nz;
+            for (int r = 0; r < P.nc; r++) {
+                if (s == P.m - 1) G.z[r] = (int)((long long)r * nz / P.nc);
+                else G.z[r] = (nz == ctx.lev[l0 + s + 1].nz ? 1 : 2) * P.lev[s + 1].z[r];
+            }
+            G.z[P.nc] = nz;
+        }
+    }
+    long long off = 0;
     for (int s = 0; s < nl; s++) {
         const Lev& L = ctx.lev[l0 + s];
-        // a row per thread at least in every loop; the tables' capacities
-        if (L.nx > SUB_TPB || nax + L.nx + L.ny + L.nz > SUB_MAX_AX || nrow + L.ny * L.nz > SUB_MAX_ROWS)
-            return false;
-        P.geo[s] = sub_geo<T>(L);
-        P.geo[s].ax0 = nax;
-        P.geo[s].row0 = nrow;
-        sub_axes<T>(L, P.ax + nax);
-        nax += L.nx + L.ny + L.nz;
-        nrow += L.ny * L.nz;
-        P.ou[s] = (int)off; off += (long long)sub_gx<T>(L) * (L.ny + 2) * (L.nz + 2);
-        P.of[s] = (int)off; off += (long long)L.nx * L.ny * L.nz;
+        ClLev<T>& G = P.lev[s];
+        G.nx = L.nx; G.ny = L.ny; G.nz = L.nz; G.nh = L.nh;
+        G.P = L.P;
+        G.gx = L.nx + 2;
+        G.gp = G.gx * (L.ny + 2);
+        int held = L.nz;  // planes of the largest share
+        if (s < P.m) {
+            held = 0;
+            for (int r = 0; r < P.nc; r++) held = std::max(held, G.z[r + 1] - G.z[r]);
+        }
+        if (s == 0 && (long long)L.nh * L.ny * held > (rows ? CL_MAX_ROWS : CL_MAX_SHARE)) return false;
+        G.uo = (int)off;
+        off += (long long)G.gp * (held + 2);
+        G.fo = (int)off;
+        off += (long long)L.nx * L.ny * held;
+        if (off * (long long)sizeof(T) > CL_SMEM_MAX) return false;
+        G.ax0 = (int)ax.size();
+        cl_axes<T>(L, G.gx, ax);
+        for (int a = 0; a < 3; a++) {
+            G.per |= L.per[a] ? 1 << a : 0;
+            G.w[a] = (T)L.w[a];
+            G.wl[a] = (T)L.wl[a];
+        }
+        G.ncol = L.nh * L.ny;
+        G.pg = std::max(1, std::min(held, CL_TPB / G.ncol));
+        G.dcol.init((unsigned)G.ncol);
+        G.dnh.init((unsigned)L.nh);
+        G.dny.init((unsigned)L.ny);
+        G.dnx.init((unsigned)L.nx);
         if (s < nl - 1) {
             const Xfer& X = ctx.xf[l0 + s];
             const int nf[3] = {L.nx, L.ny, L.nz};
             for (int a = 0; a < 3; a++) {
-                P.lin0[s][a] = nlin;
+                G.lin0[a] = (int)lin.size();
+                const Lev& C = ctx.lev[l0 + s + 1];
+                const int nc = lev_n(C, a), st = a == 0 ? 1 : (a == 1 ? C.nx + 2 : (C.nx + 2) * (C.ny + 2));
+                // coarse index x (possibly -1 or nc) -> offset and the sign of its weight
+                auto at = [&](int x, int& o) {
+                    T sgn = T(1);
+                    if (x < 0 || x >= nc) {
+                        if (C.per[a]) {
+                            if (a < 2) x = x < 0 ? nc - 1 : 0;  // along z: the ghost plane
+                        } else {
+                            if (C.bc[2 * a + (x < 0 ? 0 : 1)] == BC_DIRC) sgn = T(-1);
+                            x = x < 0 ? 0 : nc - 1;
+                        }
+                    }
+                    o = st * (x + 1);
+                    return sgn;
+                };
                 for (int i = 0; i < nf[a]; i++) {
-                    Lin e;
-                    geom_lin(X, a, i, e.j0, e.j1, e.t);
-                    P.lin[nlin + i].j0 = e.j0;
-                    P.lin[nlin + i].j1 = e.j1;
-                    P.lin[nlin + i].t = (T)e.t;
+                    ClLin<T> e;
+                    if (P.geom) {
+                        Lin b;
+                        geom_lin(X, a, i, b.j0, b.j1, b.t);
+                        e.w0 = at(b.j0, e.o0) * (T)(1.0 - b.t);
+                        e.w1 = at(b.j1, e.o1) * (T)b.t;
+                    } else if (i / 2 < nc) {
+                        const T w = (i & 1) ? T(0.125) : T(-0.125);
+                        e.w0 = at(i / 2 + 1, e.o0) * w;
+                        e.w1 = -at(i / 2 - 1, e.o1) * w;
+                    } else {  // odd last cell: not read
+                        e.o0 = e.o1 = st;
+                        e.w0 = e.w1 = T(0);
+                    }
+                    lin.push_back(e);
                 }
-                nlin += nf[a];
             }
-            // lanes per coarse cell: up to 8, while the coarse cells fill the
-            // block and a coarse row fits one trip
+            // lanes per coarse cell: up to 4 (the rows of a cell's children) while the cells leave threads idle
             const Lev& C = ctx.lev[l0 + s + 1];
-            const long long nc = (long long)C.nx * C.ny * C.nz;
-            int lg = 3;
-            while (lg > 0 && (nc << lg > SUB_TPB || (C.nx << lg) > SUB_TPB)) lg--;
-            P.rlog[s] = lg;
-            P.rrows[s] = (SUB_TPB >> lg) / C.nx;
+            const long long nc = (long long)C.nx * C.ny * ((held + 1) / 2);
+            G.rlog = nc * 4 <= CL_TPB ? 2 : (nc * 2 <= CL_TPB ? 1 : 0);
         }
-    }
-    // the solve-constant image: coefficients (ghosted), diagonal extras, inverse
-    off = (off + 1) & ~1LL;  // 16-byte boundary for either word size
-    off = ((off * (long long)sizeof(T) + 15) & ~15LL) / (long long)sizeof(T);
-    P.img_off = (int)(off * sizeof(T));
-    for (int s = 0; s < nl; s++) {
-        const Lev& L = ctx.lev[l0 + s];
-        P.ok[s] = kf ? (int)off : -1; off += kf ? (long long)sub_gx<T>(L) * (L.ny + 2) * (L.nz + 2) : 0;
-        P.od[s] = df ? (int)off : -1; off += df ? (long long)L.nx * L.ny * L.nz : 0;
     }
     size_t bytes = ((size_t)off * sizeof(T) + 15) & ~(size_t)15;
-    const Lev& Cc = ctx.lev[ctx.nlev - 1];
-    const long long ncs = (long long)Cc.nx * Cc.ny * Cc.nz;
-    P.ainv_off = ainv_in_smem ? (int)bytes : -1;
-    if (ainv_in_smem) bytes += ((size_t)(ncs * ncs) * sizeof(double) + 15) & ~(size_t)15;
-    // the tables are part of the image too (built once per solve)
-    P.lin_off = (int)bytes;
-    bytes += ((size_t)nlin * sizeof(SubLin<T>) + 15) & ~(size_t)15;
+    P.zero_vecs = (int)(bytes / 16);
+    P.stage_off = (int)bytes;
+    if (P.m > 0) {
+        const Lev& F = ctx.lev[l0 + P.m - 1];
+        const Lev& C = ctx.lev[l0 + P.m];
+        bytes += ((size_t)C.nx * C.ny * F.nz * sizeof(T) + 15) & ~(size_t)15;
+    }
+    const long long n = cells(nl - 1);
+    P.part_off = (int)bytes;
+    bytes += sizeof(double) * (size_t)std::max<long long>(CL_TPB, n);
     P.ax_off = (int)bytes;
-    bytes += ((size_t)nax * sizeof(SubAx<T>) + 15) & ~(size_t)15;
-    P.row_off = (int)bytes;
-    bytes += ((size_t)nrow * sizeof(SubRow) + 15) & ~(size_t)15;
-    P.img_bytes = (int)(bytes - P.img_off);
-    P.nlin = nlin;
-    P.nax = nax;
-    P.nrow = nrow;
-    int g = 32;
-    while (g > 1 && ncs * g > SUB_TPB) g >>= 1;
-    P.gsz = g;
+    P.nax = (int)ax.size();
+    bytes += (ax.size() * sizeof(ClAx<T>) + 15) & ~(size_t)15;
+    P.lin_off = (int)bytes;
+    P.nlin = (int)lin.size();
+    bytes += (lin.size() * sizeof(ClLin<T>) + 15) & ~(size_t)15;
     smem = bytes;
-    return bytes <= (size_t)SUB_SMEM_MAX;
+    return n <= CL_TPB && bytes <= (size_t)CL_SMEM_MAX;
 }
 
-static cudaError_t sub_launch(const void* kern, size_t smem, cudaStream_t s, void** args)
-{
-    cudaLaunchConfig_t cfg;
-    std::memset(&cfg, 0, sizeof(cfg));
-    cfg.gridDim = dim3(1);
-    cfg.blockDim = dim3(SUB_TPB);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelExC(&cfg, kern, args);
-}
-
-// build the solve-constant image of hierarchy H (after its coefficient
-// pyramid and coarsest inverse are set up); H.sub_ok tells the V-cycle
+// the cluster's part of a hierarchy: the first level whose V-cycle fits, the
+// device copy of its tables, and the row arrays of a cell coefficient's levels;
+// cl_l0 -1: none (odd periodic sizes: cells of one colour touch, and in-place
+// passes would read new values)
 template <class T>
-static int sub_image(Ctx& ctx, Hier<T>& H, const KOp<T>* ops, const mps_solver_opts* o)
+static bool cl_setup(Ctx& ctx, Hier<T>& H, const Signature& sig)
 {
-    H.sub_ok = false;
-    const int l0 = ctx.sub_l0;
-    if (l0 < 1 || !H.subimg) return 0;
-    const bool kf = ops[l0].k[0] != nullptr, df = ops[l0].dex[0] != nullptr;
-    std::unique_ptr<SubPlan<T>> pp(new SubPlan<T>);
-    SubPlan<T>& P = *pp;
+    H.cl_l0 = -1;
+    H.cltab = nullptr;
+    for (int l = 0; l < MAXL; l++) H.crow[l] = nullptr;
+    if (!ctx.sub_allowed || !cl_prepare(ctx.dev)) return true;
+    std::unique_ptr<ClPlan<T>> P(new ClPlan<T>);
+    std::vector<ClAx<T>> ax;
+    std::vector<ClLin<T>> lin;
     size_t smem = 0;
-    if (!sub_layout<T>(ctx, l0, kf, df, o, P, smem) || (size_t)P.img_bytes > H.subimg_bytes) return 0;
-    for (int s = 0; s < P.nl; s++)
-        for (int c = 0; c < 2; c++) {
-            P.k[s][c] = ops[l0 + s].k[c];
-            P.dex[s][c] = ops[l0 + s].dex[c];
+    const bool rows = sig.opclass == 1 || !sig.kuni || sig.has_reac;  // explicit rows
+    int odd = -1;  // the deepest level with an odd periodic size
+    for (int l = 0; l < ctx.nlev; l++)
+        if (odd_periodic(ctx.lev[l])) odd = l;
+    for (int l = odd + 1; l < ctx.nlev - 1; l++) {
+        if (!cl_layout<T>(ctx, l, rows, *P, smem, ax, lin)) continue;
+        H.cl_l0 = l;
+        break;
+    }
+    if (H.cl_l0 < 0) return true;
+    const size_t bytes = smem - (size_t)P->ax_off;
+    std::vector<unsigned char> img(bytes, 0);
+    std::memcpy(img.data(), ax.data(), ax.size() * sizeof(ClAx<T>));
+    if (!lin.empty())
+        std::memcpy(img.data() + (P->lin_off - P->ax_off), lin.data(), lin.size() * sizeof(ClLin<T>));
+    H.cltab = (unsigned char*)ctx.ar.get(bytes);
+    if (!H.cltab || cudaMemcpy(H.cltab, img.data(), bytes, cudaMemcpyHostToDevice) != cudaSuccess) return false;
+    if (rows)
+        for (int l = H.cl_l0; l < ctx.nlev - 1; l++) {
+            H.crow[l] = (T*)ctx.ar.get(sizeof(T) * 8 * 2 * ctx.lev[l].half);
+            if (!H.crow[l]) return false;
         }
-    const Lev& Cc = ctx.lev[ctx.nlev - 1];
-    int ncs = Cc.nx * Cc.ny * Cc.nz;
-    unsigned char* img = H.subimg;
-    const double* ainv = H.AinvT;
-    void* args[] = {(void*)&P, (void*)&img, (void*)&ainv, (void*)&ncs};
-    const void* kern = kf ? (df ? (const void*)k_sub_image<T, true, true> : (const void*)k_sub_image<T, true, false>)
-                          : (df ? (const void*)k_sub_image<T, false, true> : (const void*)k_sub_image<T, false, false>);
-    sub_launch(kern, 0, ctx.s, args);
+    return true;
+}
+
+// the explicit rows of the cluster's levels (once per solve)
+template <class T, class Op>
+static int cl_rows(Ctx& ctx, Hier<T>& H, const Op* ops)
+{
+    if (H.cl_l0 < 0 || !H.crow[H.cl_l0]) return 0;
+    std::unique_ptr<CRowsPlan<T, Op>> pp(new CRowsPlan<T, Op>);
+    CRowsPlan<T, Op>& P = *pp;
+    std::memset((void*)&P, 0, sizeof(P));
+    for (int l = H.cl_l0; l < ctx.nlev - 1; l++) {
+        const Lev& L = ctx.lev[l];
+        P.L[P.n] = L;
+        P.op[P.n] = ops[l];
+        P.rows[P.n] = H.crow[l];
+        P.blk0[P.n + 1] = P.blk0[P.n] + nblk(2 * L.half);
+        P.n++;
+    }
+    pdl_launch(k_crows<T, Op>, P.blk0[P.n], TPB, 0, ctx.s, P);
     CKL();
-    H.sub_ok = true;
     return 0;
 }
 
-// the V-cycle from level l0 (zero guess) to the coarsest and back in one
-// launch; -1 when it does not apply (the per-level launches run instead)
-template <class T>
-static int subcycle(Ctx& ctx, Hier<T>& H, const KOp<T>* ops, int l0, const mps_solver_opts* o)
+static double pass_omega(bool relaxed, int l, const mps_solver_opts* o, bool pre, int sw, int c);
+
+// the V-cycle from level H.cl_l0 to the coarsest and back in one launch
+template <class T, class Op>
+static int cluster_cycle(Ctx& ctx, Hier<T>& H, const Op* ops, const mps_solver_opts* o, bool zero_guess)
 {
-    if (!H.sub_ok || l0 != ctx.sub_l0) return -1;
-    const bool kf = ops[l0].k[0] != nullptr, df = ops[l0].dex[0] != nullptr;
-    std::unique_ptr<SubPlan<T>> pp(new SubPlan<T>);  // the kernel parameter (copied at launch)
-    SubPlan<T>& P = *pp;
+    const int l0 = H.cl_l0;
+    std::unique_ptr<ClPlan<T>> pp(new ClPlan<T>);  // the kernel parameter (copied at launch)
+    ClPlan<T>& P = *pp;
+    std::vector<ClAx<T>> ax;
+    std::vector<ClLin<T>> lin;
     size_t smem = 0;
-    if (!sub_layout<T>(ctx, l0, kf, df, o, P, smem)) return -1;
-    P.kc = ops[l0].kc;
-    P.dexc = ops[l0].dexc;
+    const bool rows = H.crow[l0] != nullptr;
+    if (!cl_layout<T>(ctx, l0, rows, P, smem, ax, lin)) {
+        ctx.err.msg = "cluster plan";
+        return MPS_ERR_CUDA;
+    }
+    P.nu1 = o->nu1;
+    P.nu2 = o->nu2;
+    P.only_black = o->nu2 >= 1;
+    P.load_u = !zero_guess;
+    for (int s = 0; s < P.nl; s++) {
+        const int l = l0 + s;
+        P.lev[s].om0 = (T)pass_omega(ctx.relaxed, l, o, true, 0, 0);
+        P.lev[s].om1 = (T)pass_omega(ctx.relaxed, l, o, false, 0, 1);
+        P.lev[s].half = ctx.lev[l].half;
+        P.lev[s].rows = H.crow[l];
+    }
+    if constexpr (std::is_same<Op, KOp<T>>::value) {
+        P.kc = ops[l0].kc;
+        P.dexc = ops[l0].dexc;
+    }
     CSplit<T> fin = csplit<T>(H.F[l0], ctx.lev[l0]);
     Split<T> uout = cur(H, ctx.lev[l0], l0);
-    const uint4* img = reinterpret_cast<const uint4*>(H.subimg);
+    const unsigned char* tab = H.cltab;
     const double* ainv = H.AinvT;
-    void* args[] = {(void*)&P, (void*)&fin, (void*)&uout, (void*)&img, (void*)&ainv};
-    const void* kern = kf ? (df ? (const void*)k_subcycle<T, true, true> : (const void*)k_subcycle<T, true, false>)
-                          : (df ? (const void*)k_subcycle<T, false, true> : (const void*)k_subcycle<T, false, false>);
-    sub_launch(kern, smem, ctx.s, args);
+    void* args[] = {(void*)&P, (void*)&fin, (void*)&uout, (void*)&tab, (void*)&ainv};
+    const void* kern = rows ? (const void*)k_cluster<T, true> : (const void*)k_cluster<T, false>;
+    cudaLaunchConfig_t cfg;
+    std::memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = dim3((unsigned)P.nc);
+    cfg.blockDim = dim3(CL_TPB);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = ctx.s;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = (unsigned)P.nc;
+    at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 2;
+    cudaLaunchKernelExC(&cfg, kern, args);
     CKL();
     return 0;
 }
@@ -1329,12 +1364,7 @@ template <class T, class Op>
 static int vcycle_rec(Ctx& ctx, Hier<T>& H, const Op* ops, int l, const mps_solver_opts* o, bool zero_guess)
 {
     if (l == ctx.nlev - 1) return coarse_solve(ctx, H, l);
-    if constexpr (std::is_same<Op, KOp<T>>::value) {
-        if (zero_guess && l == ctx.sub_l0) {
-            const int st = subcycle(ctx, H, ops, l, o);
-            if (st >= 0) return st;
-        }
-    }
+    if (l == H.cl_l0) return cluster_cycle(ctx, H, ops, o, zero_guess);
     const Lev& L = ctx.lev[l];
     const Lev& C = ctx.lev[l + 1];
     int st;
@@ -1359,12 +1389,12 @@ static int vcycle_rec(Ctx& ctx, Hier<T>& H, const Op* ops, int l, const mps_solv
     if (l == ctx.prof.level) prof_begin(ctx, MPS_PROF_RESTRICT);
     // the coarse level's first red pass from zero comes with its right-hand
     // side (cell-coefficient operators; not for the coarsest level, a level
-    // the one-block sub-cycle takes, or from the finest level, whose
+    // the cluster takes, or from the finest level, whose
     // restriction has no registers to spare: the launches below pass rz only
     // to the forms that write it and then set the level's flag)
     RedZ<T> rz{nullptr, nullptr};
     if constexpr (std::is_same<Op, KOp<T>>::value) {
-        if (l >= 1 && o->nu1 >= 1 && l + 1 < ctx.nlev - 1 && H.D[l + 1] && !(l + 1 == ctx.sub_l0 && H.sub_ok)) {
+        if (l >= 1 && o->nu1 >= 1 && l + 1 < ctx.nlev - 1 && H.D[l + 1] && l + 1 != H.cl_l0) {
             rz.u = H.U[l + 1][H.ri[l + 1] ^ 1];
             rz.d = H.D[l + 1];
         }
@@ -1614,28 +1644,9 @@ static int setup_workspace(Ctx& ctx, const Signature& sig, const mps_solver_opts
     ctx.rb.out = (double*)ctx.ar.get(sizeof(double) * 4);
     ok = ok && ctx.x64 && ctx.b64 && ctx.dense && ctx.gjM && ctx.dstatus && ctx.rb.partial && ctx.rb.counter &&
          ctx.rb.out;
-    // the one-block sub-cycle of the small levels: its first level and the
-    // solve-constant images of both hierarchies
-    ctx.sub_l0 = sig.opclass == 0 && ctx.sub_allowed && sub_prepare(ctx.dev) ? sub_first_level(ctx, o) : -1;
-    ctx.h64.subimg = nullptr;
-    ctx.h32.subimg = nullptr;
-    ctx.h64.subimg_bytes = ctx.h32.subimg_bytes = 0;
-    ctx.h64.sub_ok = ctx.h32.sub_ok = false;
-    if (ctx.sub_l0 > 0) {
-        std::unique_ptr<SubPlan<double>> p64(new SubPlan<double>);
-        std::unique_ptr<SubPlan<float>> p32(new SubPlan<float>);
-        size_t sm = 0;
-        if (need64 && sub_layout<double>(ctx, ctx.sub_l0, !sig.kuni, sig.has_reac != 0, o, *p64, sm)) {
-            ctx.h64.subimg_bytes = (size_t)p64->img_bytes;
-            ctx.h64.subimg = (unsigned char*)ctx.ar.get(ctx.h64.subimg_bytes);
-            ok = ok && ctx.h64.subimg;
-        }
-        if (need32 && sub_layout<float>(ctx, ctx.sub_l0, !sig.kuni, sig.has_reac != 0, o, *p32, sm)) {
-            ctx.h32.subimg_bytes = (size_t)p32->img_bytes;
-            ctx.h32.subimg = (unsigned char*)ctx.ar.get(ctx.h32.subimg_bytes);
-            ok = ok && ctx.h32.subimg;
-        }
-    }
+    // the small levels in one cluster
+    if (need64) ok = ok && cl_setup<double>(ctx, ctx.h64, sig);
+    if (need32) ok = ok && cl_setup<float>(ctx, ctx.h32, sig);
     if (!ok) {
         ctx.ar.clear();
         ctx.err.code = MPS_ERR_NOMEM;
@@ -2020,15 +2031,17 @@ static int solve_impl(Ctx& ctx, const mps_grid* g, int timederiv, double dt, con
         else st = coarse_inverse(ctx, ctx.h32, ctx.h32.rop[nl - 1]);
     }
     if (st) return st;
-    if (sig.opclass == 0 && !prepare_only) {  // the one-block sub-cycle's solve-constant image
-        if (need64) st = sub_image(ctx, ctx.h64, ctx.h64.kop, o);
-        else st = sub_image(ctx, ctx.h32, ctx.h32.kop, o);
+    if (!prepare_only) {  // the rows of the cluster's levels
+        if (sig.opclass == 0) st = need64 ? cl_rows(ctx, ctx.h64, ctx.h64.kop) : cl_rows(ctx, ctx.h32, ctx.h32.kop);
+        else st = need64 ? cl_rows(ctx, ctx.h64, ctx.h64.rop) : cl_rows(ctx, ctx.h32, ctx.h32.rop);
         if (st) return st;
+    }
+    if (sig.opclass == 0 && !prepare_only) {
         // the red rows' diagonals of the levels with their own launches (the
         // restriction into such a level also writes its first red pass)
         auto diag_red = [&](auto& H) -> int {
             using TT = typename std::remove_reference<decltype(*H.D[0])>::type;
-            const int lend = (ctx.sub_l0 > 0 && H.sub_ok) ? ctx.sub_l0 : nl - 1;
+            const int lend = H.cl_l0 >= 0 ? H.cl_l0 : nl - 1;
             for (int l = 1; l < lend && l < nl - 1; l++) {
                 if (!H.D[l]) continue;
                 const Lev& Ll = ctx.lev[l];
@@ -2134,7 +2147,7 @@ static int solve_impl(Ctx& ctx, const mps_grid* g, int timederiv, double dt, con
         bool red_ready = false;
         auto residual = [&]() -> int {
             Split<float> r32 = split<float>(H.F[0], L);
-            float* ured = o->nu1 >= 1 ? H.U[0][H.ri[0] ^ 1] : nullptr;
+            float* ured = o->nu1 >= 1 && H.cl_l0 != 0 ? H.U[0][H.ri[0] ^ 1] : nullptr;
             if (sig.opclass == 0)
                 return resid_norm(ctx, ctx.kop64, csplit<double>(ctx.x64, L), csplit<double>(ctx.b64, L), r32, ured,
                                   &red_ready, pass_omega(ctx.relaxed, 0, o, true, 0, 0));
@@ -2417,7 +2430,7 @@ int mps_create(mps_handle* h, int device)
     // the shared-memory (TMA) kernels and the register-fed ones give the same
     // results; the variable selects the register-fed ones (for comparisons)
     if (const char* tv = std::getenv("MPS_TMA")) ctx.tma_allowed = std::atoi(tv) != 0;
-    // the one-block sub-cycle of the small levels and the per-level launches
+    // the cluster form of the small levels and the per-level launches
     // solve the same systems; the variable selects the per-level launches
     if (const char* sv = std::getenv("MPS_SUBCYCLE")) ctx.sub_allowed = std::atoi(sv) != 0;
     if (cudaDeviceGetAttribute(&ctx.nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || ctx.nsm < 1) {
