@@ -187,12 +187,12 @@ struct Prof {
 // that is baked into its kernel parameters
 struct GraphKey {
     Signature sig;
-    int kind = -1, prec = -1, inner = 0, nu1 = 0, nu2 = 0, nlev = 0, flux = 0, transpose = 0, prof = 0, relaxed = 0;
+    int kind = -1, prec = -1, inner = 0, nu1 = 0, nu2 = 0, nlev = 0, flux = 0, transpose = 0, prof = 0, relaxed = 0, kseg = 0;
     double kc = 0, dexc = 0;
     const void* ws = nullptr;  // workspace identity (first arena block)
     bool operator==(const GraphKey& o) const
     {
-        return sig == o.sig && relaxed == o.relaxed && kind == o.kind && prec == o.prec && inner == o.inner && nu1 == o.nu1 &&
+        return sig == o.sig && relaxed == o.relaxed && kseg == o.kseg && kind == o.kind && prec == o.prec && inner == o.inner && nu1 == o.nu1 &&
                nu2 == o.nu2 && nlev == o.nlev && flux == o.flux && transpose == o.transpose && prof == o.prof &&
                kc == o.kc &&
                dexc == o.dexc && ws == o.ws;
@@ -247,6 +247,8 @@ struct Ctx {
     // FP64 coefficient pyramid (split cell fields)
     double* pk[MAXL] = {};
     double* pka[MAXL] = {};   // arithmetic means of the finest coefficient (levels >= 1; k_restrict_coef)
+    double* seg64[MAXL] = {};  // uniform segments of the coefficient on the large levels (k_kseg)
+    float* seg32[MAXL] = {};
     double* preac[MAXL] = {};
     double* pv[3][MAXL] = {};
     double* dex64[MAXL] = {};
@@ -258,6 +260,7 @@ struct Ctx {
     Hier<float> h32;
     double* x64 = nullptr;  // outer iterate (mixed / fgmres)
     double* b64 = nullptr;
+    bool kseg = false;        // this solve's operators carry the segments
     KOp<double> kop64;      // fine-level FP64 operator for outer residuals
     ROp<double> rop64;
     double* dense = nullptr;
@@ -727,23 +730,23 @@ static RestrictSplit make_restrict_split(const Lev& F, const Lev& C, const Box& 
 #ifndef MPS_TMA_LEVELS
 #define MPS_TMA_LEVELS 1  // the finest level only
 #endif
-// tile rows and blocks per SM of the FP32 pass, measured on the 257^3 mixed
-// solve (ms): 6 rows at 3 blocks per SM 12.72-12.75, 8 rows at 2 blocks
-// 12.79-12.81, 5 rows at 4 blocks 13.40, 7 rows at 3 blocks 13.78
-#ifndef MPS_TMA_BPS
-#define MPS_TMA_BPS 3  // blocks per SM the tiling aims at
-#endif
-#ifndef MPS_TMA_TJ32
-#define MPS_TMA_TJ32 6
-#endif
-#ifndef MPS_TMA_TJ64
-#define MPS_TMA_TJ64 4
-#endif
-template <class T>
-struct TmaShape {  // rows per block, one warp each; cells per thread
-    static constexpr int TJ = sizeof(T) == 4 ? MPS_TMA_TJ32 : MPS_TMA_TJ64;
+// tile rows and blocks per SM of the FP32 pass.  With a staged coefficient
+// (257^3 mixed plasma solve, ms): 6 rows at 3 blocks per SM 12.72-12.75, 8 rows
+// at 2 blocks 12.79-12.81, 5 rows at 4 blocks 13.40, 7 rows at 3 blocks 13.78.
+// Without one (uniform, or uniform along most segments; 257^3 Poisson / plasma,
+// ms): 6 rows at 3, 4, 5 blocks - / 10.73, 5.39 / 10.37, - / 10.56; 7 rows at 4
+// blocks 5.48 / 10.86, 8 rows at 4 blocks 5.13 / 10.40
+template <class T, bool KF>
+struct TmaShape {  // rows per block, one warp each; blocks per SM the tiling aims at; cells per thread
+    static constexpr int TJ = sizeof(T) == 8 ? 4 : (KF ? 6 : 8);
+    static constexpr int BPS = KF ? 3 : 4;
     static constexpr int W = 4;
 };
+// planes of a tile's chunk at least: one of fewer spends its time filling the
+// slots, and the register-fed pass is faster (129^3 mixed plasma / Poisson
+// solve, 5 planes: 3.27 / 1.69 ms against 3.47 / 1.78; 193^3 Poisson, 8 planes:
+// 3.24 against 3.10)
+constexpr int TMA_PLANES = 8;
 
 static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder()
 {
@@ -781,17 +784,17 @@ static bool encode_half(CUtensorMap* m, const T* base, const Lev& L, int rows)
 // the finest level's colour pass from a valid state with k_colour_tma;
 // returns 1 when the pass was launched, 0 when this level or operator does
 // not qualify (the caller runs the register-fed pass), < 0 on an error
-template <class T>
-static int colour_pass_tma(Ctx& ctx, Hier<T>& H, const KOp<T>& op, int l, int c, T* out, const T* fh, T om)
+template <class T, bool KF>
+static int colour_pass_tma_kf(Ctx& ctx, Hier<T>& H, const KOp<T>& op, int l, int c, T* out, const T* fh, T om)
 {
-    constexpr int TJ = TmaShape<T>::TJ, W = TmaShape<T>::W;
+    constexpr int TJ = TmaShape<T, KF>::TJ, W = TmaShape<T, KF>::W;
+    constexpr bool kf = KF;
     const Lev& L = ctx.lev[l];
     // FP32 only: the FP64 pass measured slower through shared memory (104-117
     // against 87 us at 257^3), the FP32 pass faster (49.6 against 51.2 us)
     if (sizeof(T) != 4 || !ctx.tma_ok || L.P > 256 || op.dex[0] || L.ny < 3 || L.nz < 3) return 0;
     ColourSplit cs;
     if (!make_split(L, W, cs)) return 0;
-    const bool kf = op.k[0] != nullptr;
     const int oc = c ^ 1;
     const T* uo = oc == 0 ? H.U[l][H.ri[l]] : H.U[l][H.bi[l]] + L.half;
     CUtensorMap mU, mKo, mKc, mF;
@@ -810,7 +813,7 @@ static int colour_pass_tma(Ctx& ctx, Hier<T>& H, const KOp<T>& op, int l, int c,
     // tiles for the blocks that fit on an SM (shared memory, threads, at most
     // MPS_TMA_BPS): each tile streams its planes plus two halo planes, so
     // more tiles re-read more
-    const int bps = std::max(1, std::min({(int)(227 * 1024 / (smem + 1024)), 2048 / (TJ * 32), MPS_TMA_BPS}));
+    const int bps = std::max(1, std::min({(int)(227 * 1024 / (smem + 1024)), 2048 / (TJ * 32), TmaShape<T, KF>::BPS}));
     // the interior box of the split: rows 1 .. jhi, planes 1 .. khi (one cell
     // short of merged last cells); the shell blocks take every other row
     tc.jhi = cs.b.hi[1];
@@ -819,6 +822,7 @@ static int colour_pass_tma(Ctx& ctx, Hier<T>& H, const KOp<T>& op, int l, int c,
     tc.njb = (tc.jhi + TJ - 1) / TJ;
     const int want = std::max(1, ctx.nsm * bps / tc.njb);
     tc.tk = std::max(1, (tc.khi + want - 1) / want);
+    if (tc.tk < TMA_PLANES) return 0;
     tc.nkb = (tc.khi + tc.tk - 1) / tc.tk;
     tc.ntile = tc.njb * tc.nkb;
     tc.g_lo = cs.g_lo;
@@ -838,8 +842,15 @@ static int colour_pass_tma(Ctx& ctx, Hier<T>& H, const KOp<T>& op, int l, int c,
         }
         return 1;
     };
-    if (L.uniform) return kf ? launch(k_colour_tma<T, W, TJ, true, true>) : launch(k_colour_tma<T, W, TJ, false, true>);
-    return kf ? launch(k_colour_tma<T, W, TJ, true, false>) : launch(k_colour_tma<T, W, TJ, false, false>);
+    if (L.uniform) return launch(k_colour_tma<T, W, TJ, KF, true>);
+    return launch(k_colour_tma<T, W, TJ, KF, false>);
+}
+template <class T>
+static int colour_pass_tma(Ctx& ctx, Hier<T>& H, const KOp<T>& op, int l, int c, T* out, const T* fh, T om)
+{
+    // (a coefficient with uniform segments is not staged)
+    if (op.k[0] && !op.seg) return colour_pass_tma_kf<T, true>(ctx, H, op, l, c, out, fh, om);
+    return colour_pass_tma_kf<T, false>(ctx, H, op, l, c, out, fh, om);
 }
 
 // the attributes the shared-memory colour pass needs, set outside any stream
@@ -853,12 +864,9 @@ static bool tma_prepare(int dev)
         auto set = [&](auto kern) {
             return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess;
         };
-        constexpr int W32 = TmaShape<float>::W, J32 = TmaShape<float>::TJ;
-        constexpr int W64 = TmaShape<double>::W, J64 = TmaShape<double>::TJ;
-        bool ok = set(k_colour_tma<float, W32, J32, true, true>) && set(k_colour_tma<float, W32, J32, false, true>) &&
-                  set(k_colour_tma<float, W32, J32, true, false>) && set(k_colour_tma<float, W32, J32, false, false>) &&
-                  set(k_colour_tma<double, W64, J64, true, true>) && set(k_colour_tma<double, W64, J64, false, true>) &&
-                  set(k_colour_tma<double, W64, J64, true, false>) && set(k_colour_tma<double, W64, J64, false, false>);
+        constexpr int W = TmaShape<float, true>::W, JK = TmaShape<float, true>::TJ, JU = TmaShape<float, false>::TJ;
+        bool ok = set(k_colour_tma<float, W, JK, true, true>) && set(k_colour_tma<float, W, JU, false, true>) &&
+                  set(k_colour_tma<float, W, JK, true, false>) && set(k_colour_tma<float, W, JU, false, false>);
         if (!ok) cudaGetLastError();
         return ok;
     });
@@ -1603,6 +1611,14 @@ static void alloc_hier(Ctx& ctx, Hier<T>& H, bool& ok)
     ok = ok && H.AinvT && H.Dprev && H.gj;
 }
 
+// levels whose coefficient is described by uniform segments where it can be:
+// those bound by bytes (a smaller level's passes are bound by latency, which the
+// segment's own load would lengthen).  257^3 plasma solve without / on the finest
+// level / on the finest two: 11.80 / 10.79 / 10.73 ms mixed, 18.0 / 15.52 / 15.44 ms
+// FP64; the 129^3 step 5.58 / 5.51 / 5.51 ms
+constexpr long long SEG_MIN_CELLS = 1 << 19;
+static bool seg_level(const Lev& L) { return (long long)L.nx * L.ny * L.nz >= SEG_MIN_CELLS && L.nx >= 32; }
+
 static int setup_workspace(Ctx& ctx, const Signature& sig, const mps_solver_opts* o, int need64, int need32)
 {
     if (sig == ctx.sig) return 0;
@@ -1625,6 +1641,11 @@ static int setup_workspace(Ctx& ctx, const Signature& sig, const mps_solver_opts
             ctx.rows32[l] = need32 ? (float*)ctx.ar.get(7 * b32) : nullptr;
         } else {
             ctx.k32[l] = (need32 && !sig.kuni) ? (float*)ctx.ar.get(b32) : nullptr;
+            const bool segs = !sig.kuni && seg_level(L);
+            const size_t ns = (size_t)L.rows * ((L.nh + 15) / 16);
+            ctx.seg64[l] = segs ? (double*)ctx.ar.get(sizeof(double) * ns) : nullptr;
+            ctx.seg32[l] = segs ? (float*)ctx.ar.get(sizeof(float) * ns) : nullptr;
+            ok = ok && (!segs || (ctx.seg64[l] && ctx.seg32[l]));
             ctx.dex32[l] = (need32 && sig.has_reac) ? (float*)ctx.ar.get(b32) : nullptr;
         }
     }
@@ -1704,6 +1725,8 @@ static void set_kop(Ctx& ctx, KOp<T>* ops, T* const* kT, T* const* dexT, double 
     for (int l = 0; l < ctx.nlev; l++) {
         const Lev& L = ctx.lev[l];
         KOp<T> op;
+        op.seg = nullptr;
+        op.nseg = 0;
         if (kuni) { op.k[0] = op.k[1] = nullptr; op.kc = (T)kc; }
         else { op.k[0] = kT[l]; op.k[1] = kT[l] + L.half; op.kc = T(0); }
         if (has_reac) { op.dex[0] = dexT[l]; op.dex[1] = dexT[l] + L.half; op.dexc = T(0); }
@@ -1978,9 +2001,31 @@ static int solve_impl(Ctx& ctx, const mps_grid* g, int timederiv, double dt, con
         }
         KOp<double> k64[MAXL];
         set_kop<double>(ctx, k64, ctx.pk, ctx.dex64, k0, dtinv, sig.kuni, sig.has_reac);
+        if (need32) set_kop<float>(ctx, ctx.h32.kop, ctx.k32, ctx.dex32, k0, dtinv, sig.kuni, sig.has_reac);
+        // a coefficient that is constant along most segments: at most one change in
+        // four 32-cell chunks of the rows, and in a quarter of the sampled columns
+        // (four a row) from row to row (the passes then read one word for 32 cells;
+        // where most segments differ, that word is one more)
+        const unsigned long long nchunk = (unsigned long long)L0.rows * (unsigned)((L0.nx + 31) / 32);
+        ctx.kseg = !prepare_only && !sig.kuni && hm[6] <= nchunk / 4 && hm[7] <= (unsigned long long)L0.rows;
+        if (ctx.kseg) {
+            auto segments = [&](auto* k, auto* seg, auto& op, int l) -> int {
+                using TT = typename std::remove_pointer<decltype(seg)>::type;
+                const Lev& L = ctx.lev[l];
+                op.seg = seg;
+                op.nseg = (L.nh + 15) / 16;
+                const long long nw = (long long)L.rows * ((op.nseg + 1) / 2);
+                pdl_launch(k_kseg<TT>, nblk(32 * nw), TPB, 0, ctx.s, L, csplit<TT>(k, L), seg, op.nseg);
+                CKL();
+                return 0;
+            };
+            for (int l = 0; l < nl && ctx.seg64[l]; l++) {
+                if ((need64 || l == 0) && (st = segments(ctx.pk[l], ctx.seg64[l], k64[l], l))) return st;
+                if (need32 && (st = segments(ctx.k32[l], ctx.seg32[l], ctx.h32.kop[l], l))) return st;
+            }
+        }
         ctx.kop64 = k64[0];
         if (need64) std::copy(k64, k64 + nl, ctx.h64.kop);
-        if (need32) set_kop<float>(ctx, ctx.h32.kop, ctx.k32, ctx.dex32, k0, dtinv, sig.kuni, sig.has_reac);
     } else {
         for (int l = 0; l < nl; l++) {
             if (ctx.rows64[l] && (need64 || l == 0)) {
@@ -2086,6 +2131,7 @@ static int solve_impl(Ctx& ctx, const mps_grid* g, int timederiv, double dt, con
     gk.dexc = sig.has_reac ? 0.0 : dtinv;
     gk.ws = ctx.ar.blocks.empty() ? nullptr : ctx.ar.blocks[0];
     gk.relaxed = ctx.relaxed;
+    gk.kseg = sig.opclass == 0 && ctx.kseg;
     gk.prof = ctx.prof.on ? 1 + ctx.prof.level : 0;  // profiled graphs carry event-record nodes
     // graphs need the buffer parities to return after one iteration
     const bool graphs = o->use_graph && ((o->nu1 + o->nu2) % 2 == 0);
