@@ -876,7 +876,7 @@ def run_ours(args, ws, rank, local):
         "hbm_gbs_solve": gbs_m,
         "hbm_frac_solve": gbs_m / hbm_peak,
         "fp64_hbm_frac_solve": gbs_d / hbm_peak,
-        "roofline": {"bound": "hbm", "kernel": "finest-level red/black pass, FP32, mixed solve: k_colour_tma<float,4,6> "
+        "roofline": {"bound": "hbm", "kernel": "finest-level red/black pass, FP32, mixed solve: k_colour_tma<float,4,8> "
                                                "(TMA-staged rows; the passes from a valid state) and "
                                                "k_colourv_split<float,4> (the black pass after each outer residual, "
                                                "which writes the red pass from zero itself), averaged",

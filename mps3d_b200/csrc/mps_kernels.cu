@@ -165,9 +165,10 @@ __global__ void k_maxabs_all(Lev L, const double* __restrict__ vel, const double
         const unsigned k = L.divNy.div(row), j = row - k * (unsigned)L.ny;
         const long long base = 1 + gx * ((long long)(j + 1) + gy * (long long)(k + 1));
         // how often the coefficient changes between the rows, on four columns of each,
-        // and along x (for the rule on uniform segments; a shuffle for the latter
+        // and along x (for the rule on uniform segments, which operators without a
+        // velocity use; a shuffle for the latter
         // holds the loads of the loop back: 222 against 100 us at 257^3)
-        if (lane < 4 && (int)lane < L.nx) {
+        if (!vel && lane < 4 && (int)lane < L.nx) {
             const long long g = base + lane;
             const double d = dcoeff[g];
             nvr += (j + 1 < (unsigned)L.ny && dcoeff[g + gx] != d) ||
@@ -176,7 +177,7 @@ __global__ void k_maxabs_all(Lev L, const double* __restrict__ vel, const double
         for (int i = lane; i < L.nx; i += 32) {
             const long long g = base + i;
             const double d = dcoeff[g];
-            nvx += dcoeff[i + 1 < L.nx ? g + 1 : g] != d;
+            if (!vel) nvx += dcoeff[i + 1 < L.nx ? g + 1 : g] != d;
             if (vel) {
                 upd(m[0], vel[g]);
                 upd(m[0], vel[g + ng]);

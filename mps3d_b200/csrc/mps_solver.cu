@@ -2011,7 +2011,7 @@ static int solve_impl(Ctx& ctx, const mps_grid* g, int timederiv, double dt, con
         // (four a row) from row to row (the passes then read one word for 32 cells;
         // where most segments differ, that word is one more)
         const unsigned long long nchunk = (unsigned long long)L0.rows * (unsigned)((L0.nx + 31) / 32);
-        ctx.kseg = !prepare_only && !sig.kuni && hm[6] <= nchunk / 4 && hm[7] <= (unsigned long long)L0.rows;
+        ctx.kseg = !prepare_only && !sig.kuni && !in.vel && hm[6] <= nchunk / 4 && hm[7] <= (unsigned long long)L0.rows;
         if (ctx.kseg) {
             auto segments = [&](auto* k, auto* seg, auto& op, int l) -> int {
                 using TT = typename std::remove_pointer<decltype(seg)>::type;
@@ -2399,7 +2399,7 @@ static int solve_impl(Ctx& ctx, const mps_grid* g, int timederiv, double dt, con
     if (ctx.prof.on) {
         prof_collect(ctx);
         ctx.prof.precision_bytes = mixed ? 4 : 8;
-        ctx.prof.coeff_field = sig.opclass == 0 ? !sig.kuni : 7;
+        ctx.prof.coeff_field = sig.opclass == 0 ? !sig.kuni && !ctx.kseg : 7;
         ctx.prof.cells = ncell;
     }
     inf.launches = (int)(ctx.launches - launches0);
