@@ -158,6 +158,8 @@ struct Hier {
     double* AinvT = nullptr;
     int cl_l0 = -1;                   // first level of the cluster's V-cycle (k_cluster), -1: none
     unsigned char* cltab = nullptr;   // its axis and interpolation tables
+    std::vector<unsigned char> climg; // the host copy of the tables on the device (cl_tables)
+    double cl_len[3] = {0, 0, 0};     // the box that they hold
     T* crow[MAXL] = {};               // explicit rows of a cell coefficient on its levels (k_krows)
     double* Dprev = nullptr;  // the coarsest matrix whose inverse AinvT holds
     int* gj = nullptr;        // its inversion state (k_gauss_jordan)
@@ -189,10 +191,11 @@ struct GraphKey {
     Signature sig;
     int kind = -1, prec = -1, inner = 0, nu1 = 0, nu2 = 0, nlev = 0, flux = 0, transpose = 0, prof = 0, relaxed = 0, kseg = 0;
     double kc = 0, dexc = 0;
+    double len[3] = {0, 0, 0};  // the box: the levels' face coefficients
     const void* ws = nullptr;  // workspace identity (first arena block)
     bool operator==(const GraphKey& o) const
     {
-        return sig == o.sig && relaxed == o.relaxed && kseg == o.kseg && kind == o.kind && prec == o.prec && inner == o.inner && nu1 == o.nu1 &&
+        return sig == o.sig && std::equal(len, len + 3, o.len) && relaxed == o.relaxed && kseg == o.kseg && kind == o.kind && prec == o.prec && inner == o.inner && nu1 == o.nu1 &&
                nu2 == o.nu2 && nlev == o.nlev && flux == o.flux && transpose == o.transpose && prof == o.prof &&
                kc == o.kc &&
                dexc == o.dexc && ws == o.ws;
@@ -239,6 +242,7 @@ struct Ctx {
     size_t inbuf_bytes = 0;
     Signature sig;
     int nlev = 0;
+    double len[3] = {0, 0, 0};  // edge lengths of the box that lev describes
     Lev lev[MAXL];
     Xfer xf[MAXL];
     Lin* dtab = nullptr;      // device prolongation tables of the current plan
@@ -1251,8 +1255,8 @@ static bool cl_layout(const Ctx& ctx, int l0, bool rows, ClPlan<T>& P, size_t& s
     return n <= CL_TPB && bytes <= (size_t)CL_SMEM_MAX;
 }
 
-// the cluster's part of a hierarchy: the first level whose V-cycle fits, the
-// device copy of its tables, and the row arrays of a cell coefficient's levels;
+// the cluster's part of a hierarchy: the first level whose V-cycle fits, room
+// for its tables, and the row arrays of its explicit rows;
 // cl_l0 -1: none (odd periodic sizes: cells of one colour touch, and in-place
 // passes would read new values)
 template <class T>
@@ -1260,6 +1264,7 @@ static bool cl_setup(Ctx& ctx, Hier<T>& H, const Signature& sig)
 {
     H.cl_l0 = -1;
     H.cltab = nullptr;
+    H.cl_len[0] = H.cl_len[1] = H.cl_len[2] = 0.0;
     for (int l = 0; l < MAXL; l++) H.crow[l] = nullptr;
     if (!ctx.sub_allowed || !cl_prepare(ctx.dev)) return true;
     std::unique_ptr<ClPlan<T>> P(new ClPlan<T>);
@@ -1276,19 +1281,38 @@ static bool cl_setup(Ctx& ctx, Hier<T>& H, const Signature& sig)
         break;
     }
     if (H.cl_l0 < 0) return true;
-    const size_t bytes = smem - (size_t)P->ax_off;
-    std::vector<unsigned char> img(bytes, 0);
-    std::memcpy(img.data(), ax.data(), ax.size() * sizeof(ClAx<T>));
-    if (!lin.empty())
-        std::memcpy(img.data() + (P->lin_off - P->ax_off), lin.data(), lin.size() * sizeof(ClLin<T>));
-    H.cltab = (unsigned char*)ctx.ar.get(bytes);
-    if (!H.cltab || cudaMemcpy(H.cltab, img.data(), bytes, cudaMemcpyHostToDevice) != cudaSuccess) return false;
+    H.cltab = (unsigned char*)ctx.ar.get(smem - (size_t)P->ax_off);
+    if (!H.cltab) return false;
     if (rows)
         for (int l = H.cl_l0; l < ctx.nlev - 1; l++) {
             H.crow[l] = (T*)ctx.ar.get(sizeof(T) * 8 * 2 * ctx.lev[l].half);
             if (!H.crow[l]) return false;
         }
     return true;
+}
+
+// the cluster's tables for the present box, in stream order.  They hold the face
+// coefficients, which scale with the box, and the workspace outlives it: the
+// tables on the device are kept while the box stays the same
+template <class T>
+static int cl_tables(Ctx& ctx, Hier<T>& H)
+{
+    if (H.cl_l0 < 0 || std::equal(ctx.len, ctx.len + 3, H.cl_len)) return 0;
+    std::unique_ptr<ClPlan<T>> P(new ClPlan<T>);
+    std::vector<ClAx<T>> ax;
+    std::vector<ClLin<T>> lin;
+    size_t smem = 0;
+    if (!cl_layout<T>(ctx, H.cl_l0, H.crow[H.cl_l0] != nullptr, *P, smem, ax, lin)) {
+        ctx.err.msg = "cluster plan";
+        return MPS_ERR_CUDA;
+    }
+    H.climg.assign(smem - (size_t)P->ax_off, 0);
+    std::memcpy(H.climg.data(), ax.data(), ax.size() * sizeof(ClAx<T>));
+    if (!lin.empty())
+        std::memcpy(H.climg.data() + (P->lin_off - P->ax_off), lin.data(), lin.size() * sizeof(ClLin<T>));
+    CK(cudaMemcpyAsync(H.cltab, H.climg.data(), H.climg.size(), cudaMemcpyHostToDevice, ctx.s));
+    std::copy(ctx.len, ctx.len + 3, H.cl_len);
+    return 0;
 }
 
 // the explicit rows of the cluster's levels (once per solve)
@@ -1839,6 +1863,9 @@ static int solve_impl(Ctx& ctx, const mps_grid* g, int timederiv, double dt, con
     int nl = plan_levels(g, o, bc, ctx.lev, ctx.xf, why);
     if (nl < 1) { ctx.err.msg = why; return MPS_ERR_BAD_ARG; }
     ctx.nlev = nl;
+    ctx.len[0] = g->llenx;
+    ctx.len[1] = g->lleny;
+    ctx.len[2] = g->llenz;
     const Lev& L0 = ctx.lev[0];
     {  // 1-D prolongation tables of the geometric transfers
         size_t total = 0;
@@ -2079,7 +2106,8 @@ static int solve_impl(Ctx& ctx, const mps_grid* g, int timederiv, double dt, con
         else st = coarse_inverse(ctx, ctx.h32, ctx.h32.rop[nl - 1]);
     }
     if (st) return st;
-    if (!prepare_only) {  // the rows of the cluster's levels
+    if (!prepare_only) {  // the tables and rows of the cluster's levels
+        if ((st = need64 ? cl_tables(ctx, ctx.h64) : cl_tables(ctx, ctx.h32))) return st;
         if (sig.opclass == 0) st = need64 ? cl_rows(ctx, ctx.h64, ctx.h64.kop) : cl_rows(ctx, ctx.h32, ctx.h32.kop);
         else st = need64 ? cl_rows(ctx, ctx.h64, ctx.h64.rop) : cl_rows(ctx, ctx.h32, ctx.h32.rop);
         if (st) return st;
@@ -2132,6 +2160,7 @@ static int solve_impl(Ctx& ctx, const mps_grid* g, int timederiv, double dt, con
     gk.transpose = sig.transpose;  // a symmetric operator's transposed solve replays the forward graphs
     gk.kc = sig.kuni ? k0 : 0.0;
     gk.dexc = sig.has_reac ? 0.0 : dtinv;
+    std::copy(ctx.len, ctx.len + 3, gk.len);
     gk.ws = ctx.ar.blocks.empty() ? nullptr : ctx.ar.blocks[0];
     gk.relaxed = ctx.relaxed;
     gk.kseg = sig.opclass == 0 && ctx.kseg;
