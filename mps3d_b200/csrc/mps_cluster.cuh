@@ -186,10 +186,13 @@ __device__ __forceinline__ void cl_begin(const ClPlan<T>& P, int s)
 
 // where a level's boundary planes are shown: a cell at ghosted index g of local
 // plane 0 (nl-1) also goes to lo (hi) + g elements, the upper (lower) ghost plane
-// of the block below (above); 0: nowhere
+// of the block below (above); CL_NOWHERE: to no block.  Each is an address less
+// the offset of the cell's own plane, so it may lie below the shared memory or
+// wrap: any multiple of the word can occur, 0 among them, an odd number cannot
 struct ClPush {
     unsigned lo, hi;
 };
+constexpr unsigned CL_NOWHERE = 1u;
 template <class T>
 __device__ __forceinline__ ClPush cl_pushes(const ClPlan<T>& P, const ClMem<T>& M, int s, int z0, int nl)
 {
@@ -197,15 +200,15 @@ __device__ __forceinline__ ClPush cl_pushes(const ClPlan<T>& P, const ClMem<T>& 
     const bool per = (G.per >> 2) & 1, one = s >= P.m;  // one: the first block holds the whole level
     const int nlo = one ? nl : G.z[M.rlo + 1] - G.z[M.rlo];
     ClPush p;
-    p.lo = z0 > 0 || per ? (one ? M.self : M.lo) + (unsigned)sizeof(T) * (unsigned)(G.uo + G.gp * nlo) : 0u;
-    p.hi = z0 + nl < G.nz || per ? (one ? M.self : M.hi) + (unsigned)sizeof(T) * (unsigned)(G.uo - G.gp * nl) : 0u;
+    p.lo = z0 > 0 || per ? (one ? M.self : M.lo) + (unsigned)sizeof(T) * (unsigned)(G.uo + G.gp * nlo) : CL_NOWHERE;
+    p.hi = z0 + nl < G.nz || per ? (one ? M.self : M.hi) + (unsigned)sizeof(T) * (unsigned)(G.uo - G.gp * nl) : CL_NOWHERE;
     return p;
 }
 template <class T>
 __device__ __forceinline__ void cl_push(const ClPush& p, int g, int kl, int nl, T v)
 {
-    if (kl == 0 && p.lo) cl_st(p.lo + (unsigned)sizeof(T) * (unsigned)g, v);
-    if (kl == nl - 1 && p.hi) cl_st(p.hi + (unsigned)sizeof(T) * (unsigned)g, v);
+    if (kl == 0 && p.lo != CL_NOWHERE) cl_st(p.lo + (unsigned)sizeof(T) * (unsigned)g, v);
+    if (kl == nl - 1 && p.hi != CL_NOWHERE) cl_st(p.hi + (unsigned)sizeof(T) * (unsigned)g, v);
 }
 
 // the explicit row of one cell: diagonal, its reciprocal, x-, x+, y-, y+, z-, z+
@@ -307,7 +310,7 @@ __device__ __forceinline__ void cl_smooth(const ClPlan<T>& P, const ClMem<T>& M,
         else om = c == 0 && sw == 0 ? T(1) : om1;
         // the last pass of all stores into no other block (they may have left)
         const bool push = pre || s > 0 || ps < 2 * nsw - 1;
-        const unsigned lo = push ? pd.lo : 0u, hi = push ? pd.hi : 0u;
+        const unsigned lo = push ? pd.lo : CL_NOWHERE, hi = push ? pd.hi : CL_NOWHERE;
         const T* rc = rows + c * rhalf;
         ClCell<T, RF> w[B];
         // no branches within a batch: a cell that does not exist takes the column's first row
@@ -366,8 +369,8 @@ __device__ __forceinline__ void cl_smooth(const ClPlan<T>& P, const ClMem<T>& M,
                     const int g = K.g0 + q + gp * (kl + 1);
                     const bool ok = exists(kl, q);
                     if (ok) u[g] = v[b];
-                    if (ok && kl == 0 && lo) cl_st(lo + (unsigned)sizeof(T) * (unsigned)g, v[b]);
-                    if (ok && kl == nl - 1 && hi) cl_st(hi + (unsigned)sizeof(T) * (unsigned)g, v[b]);
+                    if (ok && kl == 0 && lo != CL_NOWHERE) cl_st(lo + (unsigned)sizeof(T) * (unsigned)g, v[b]);
+                    if (ok && kl == nl - 1 && hi != CL_NOWHERE) cl_st(hi + (unsigned)sizeof(T) * (unsigned)g, v[b]);
                 }
             }
         }
