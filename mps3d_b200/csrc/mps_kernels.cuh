@@ -67,9 +67,12 @@ template <class T>
 __device__ __forceinline__ T own_at(const CSplit<T>& u, int c, long long o) { return __ldg(&u.half(c)[o]); }
 
 // the Gauss-Seidel value v over-relaxed from the cell's old value: om = 1 is
-// plain Gauss-Seidel (the callers then do not read the old value)
-template <class T>
-__device__ __forceinline__ T relax_to(T om, T v, T own) { return own + om * (v - own); }
+// plain Gauss-Seidel (the callers then do not read the old value).  v - own is
+// rounded by itself: left to the compiler it was fused with v's division in some
+// kernels and not in others (the staged and the register-fed pass then 5e-8 to 2e-6
+// apart after two iterations)
+__device__ __forceinline__ float relax_to(float om, float v, float own) { return fmaf(om, __fsub_rn(v, own), own); }
+__device__ __forceinline__ double relax_to(double om, double v, double own) { return fma(om, __dsub_rn(v, own), own); }
 
 // ---------------------------------------------------------------------
 // one colour pass of red-black Gauss-Seidel, out of place:
