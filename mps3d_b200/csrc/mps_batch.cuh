@@ -41,7 +41,7 @@ struct BDetect {
     unsigned rows;
     FastDiv divNy;
     int blk0, nblk;
-    unsigned long long* out;  // 9 words: k_maxabs_all's six maxima (two spare), dcoeff(1,1,1)
+    unsigned long long* out;  // DET_WORDS words, without the counts of changes
 };
 
 // the detection of every problem of a batch in one launch: each problem's
@@ -59,8 +59,9 @@ __global__ void __launch_bounds__(256) kb_detect(const BDetect* __restrict__ dd,
     const long long gx = d.nx + 2, gy = d.ny + 2;
     const long long ng = gx * gy * (d.nz + 2);
     const double ref = d.dcoeff[1 + gx * (1 + gy)];
-    if (blockIdx.x == (unsigned)d.blk0 && threadIdx.x == 0) d.out[8] = (unsigned long long)__double_as_longlong(ref);
+    if (blockIdx.x == (unsigned)d.blk0 && threadIdx.x == 0) d.out[DET_REF] = (unsigned long long)__double_as_longlong(ref);
     long long m[6] = {0, 0, 0, 0, 0, 0};
+    unsigned long long top = 0;
     auto upd = [](long long& cur, double v) {
         v = fabs(v);
         if (!(v <= 1.0e308)) v = __longlong_as_double(0x7ff8000000000000LL);
@@ -79,7 +80,10 @@ __global__ void __launch_bounds__(256) kb_detect(const BDetect* __restrict__ dd,
                 upd(m[0], d.vel[g + ng]);
                 upd(m[0], d.vel[g + 2 * ng]);
             }
-            if (d.reac) upd(m[1], d.reac[g]);
+            if (d.reac) {
+                upd(m[1], d.reac[g]);
+                top = max(top, ordered_key(__double_as_longlong(d.reac[g])));
+            }
             const double c = d.dcoeff[g];
             upd(m[2], c - ref);
             upd(m[5], c);
@@ -96,6 +100,7 @@ __global__ void __launch_bounds__(256) kb_detect(const BDetect* __restrict__ dd,
         }
         if (lane == 0 && b > 0) atomicMax(d.out + q, (unsigned long long)b);
     }
+    if (d.reac) reduce_top(top, d.out + DET_REAC);
 }
 
 // every problem active, no iteration done (the start of a batched solve)
@@ -583,7 +588,7 @@ struct BatchState {
     std::vector<long long> tune_key;
     std::vector<int> tune_grid;
     std::vector<int> tune_vec;
-    // operator detection of every problem (9 words each), read back at once
+    // operator detection of every problem (DET_WORDS each), read back at once
     unsigned long long* ddet = nullptr;
     unsigned long long* hdet = nullptr;  // page-locked
     BDetect* ddd = nullptr;              // the detection launch's problem table
@@ -626,7 +631,7 @@ static int sub_init(Ctx& parent, Ctx& sc)
     sc.sub_allowed = false;  // the batched steps run every level themselves
     if (cudaEventCreate(&sc.e0) != cudaSuccess || cudaEventCreate(&sc.e1) != cudaSuccess ||
         cudaMallocHost((void**)&sc.hpin, sizeof(double) * 512) != cudaSuccess ||
-        cudaMalloc((void**)&sc.dmax, sizeof(unsigned long long) * 8) != cudaSuccess)
+        cudaMalloc((void**)&sc.dmax, sizeof(unsigned long long) * DET_WORDS) != cudaSuccess)
         return MPS_ERR_CUDA;
     return MPS_OK;
 }
@@ -1119,8 +1124,8 @@ static std::vector<long long> prep_key_of(int wordsize, int np, const mps_proble
         bytes(&probs[p], sizeof(mps_problem));
         k.push_back(scanned[p]);
         if (scanned[p]) {
-            double v[9];
-            std::memcpy(v, det + 9 * p, sizeof(v));
+            double v[DET_WORDS];
+            std::memcpy(v, det + (size_t)DET_WORDS * p, sizeof(v));
             bool finite = true;
             for (int q = 0; q < 6; q++) finite = finite && v[q] <= 1e308;
             const bool kuni = v[2] == 0.0;
@@ -1130,8 +1135,20 @@ static std::vector<long long> prep_key_of(int wordsize, int np, const mps_proble
             k.push_back(kuni);
             k.push_back(v[4] == 0.0);  // zero initial guess
             long long kb = 0;
-            if (kuni) std::memcpy(&kb, &v[8], 8);  // the uniform coefficient enters the operators
+            if (kuni) std::memcpy(&kb, &v[DET_REF], 8);  // the uniform coefficient enters the operators
             k.push_back(kb);
+            // the levels with over-relaxed passes
+            const mps_problem& q = probs[p];
+            const double dmin = diag_extra_min(q.timederiv && q.dt > 0 ? 1.0 / q.dt : 0.0, v[1],
+                                               det[(size_t)DET_WORDS * p + DET_REAC]);
+            int nrel = MAXL;
+            if (dmin > 0 && o->hierarchy == MPS_HIER_GEOM) {
+                Lev lev[MAXL];
+                Xfer xf[MAXL];
+                std::string why;
+                nrel = relaxed_levels(lev, plan_levels(&q.g, o, q.bc_code, lev, xf, why), dmin, v[5]);
+            }
+            k.push_back(nrel);
         }
     }
     return k;
@@ -1170,8 +1187,8 @@ static int batched_solve(Ctx& ctx, int np, const mps_problem* probs, const mps_s
         B.ddd = nullptr;
         B.hdd = nullptr;
         B.det_cap = 0;
-        if (cudaMalloc((void**)&B.ddet, sizeof(unsigned long long) * 9 * np) != cudaSuccess ||
-            cudaMallocHost((void**)&B.hdet, sizeof(unsigned long long) * 9 * np) != cudaSuccess ||
+        if (cudaMalloc((void**)&B.ddet, sizeof(unsigned long long) * DET_WORDS * np) != cudaSuccess ||
+            cudaMallocHost((void**)&B.hdet, sizeof(unsigned long long) * DET_WORDS * np) != cudaSuccess ||
             cudaMalloc((void**)&B.ddd, sizeof(BDetect) * np) != cudaSuccess ||
             cudaMallocHost((void**)&B.hdd, sizeof(BDetect) * np) != cudaSuccess) {
             ctx.err.msg = "batched: detection buffers";
@@ -1203,17 +1220,17 @@ static int batched_solve(Ctx& ctx, int np, const mps_problem* probs, const mps_s
         d.divNy.init((unsigned)g.ly);
         d.blk0 = blocks;
         d.nblk = (int)std::min<long long>(((long long)d.rows + 7) / 8, 256);  // a warp per row, 8 per block
-        d.out = B.ddet + 9 * p;
+        d.out = B.ddet + (size_t)DET_WORDS * p;
         blocks += d.nblk;
         scanned[p] = 1;
     }
-    CK(cudaMemsetAsync(B.ddet, 0, sizeof(unsigned long long) * 9 * np, ctx.s));
+    CK(cudaMemsetAsync(B.ddet, 0, sizeof(unsigned long long) * DET_WORDS * np, ctx.s));
     if (ndet > 0) {
         CK(cudaMemcpyAsync(B.ddd, B.hdd, sizeof(BDetect) * ndet, cudaMemcpyHostToDevice, ctx.s));
         kb_detect<<<blocks, 256, 0, ctx.s>>>(B.ddd, ndet);
         CKL();
     }
-    CK(cudaMemcpyAsync(B.hdet, B.ddet, sizeof(unsigned long long) * 9 * np, cudaMemcpyDeviceToHost, ctx.s));
+    CK(cudaMemcpyAsync(B.hdet, B.ddet, sizeof(unsigned long long) * DET_WORDS * np, cudaMemcpyDeviceToHost, ctx.s));
     CK(cudaStreamSynchronize(ctx.s));
     // the set-up of every problem: run eagerly, captured as a graph at the
     // second call with the same key (then launched), or replayed
@@ -1252,7 +1269,7 @@ static int batched_solve(Ctx& ctx, int np, const mps_problem* probs, const mps_s
             mps_solve_info inf;
             sc.launches = 0;
             int st = solve_impl(sc, &q.g, q.timederiv, q.dt, in, q.bc_code, o, &inf, 0, 1,
-                                scanned[p] ? B.hdet + 9 * p : nullptr);
+                                scanned[p] ? B.hdet + (size_t)DET_WORDS * p : nullptr);
             ctx.launches += sc.launches;
             if (st) {
                 ctx.err.msg = "batched problem " + std::to_string(p) + ": " + sc.err.msg;

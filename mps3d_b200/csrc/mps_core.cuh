@@ -186,6 +186,22 @@ struct KOp {
     const T* seg;
     int nseg;  // segments per row
 };
+// The words of an operator detection: largest magnitudes of the velocity, the
+// reaction, the coefficient less its first cell's, the source, the guess and the
+// coefficient; how often the coefficient changes along x and between rows (single
+// solves without a velocity); the first cell's coefficient (batched solves); the
+// largest reaction, signed (ordered_key; 0 without a reaction field).
+constexpr int DET_REF = 8, DET_REAC = 9, DET_WORDS = 10;
+// a key whose unsigned order is the doubles' order, never 0 for a finite value
+__host__ __device__ inline unsigned long long ordered_key(long long b)
+{
+    return b < 0 ? ~(unsigned long long)b : (unsigned long long)b | 1ull << 63;
+}
+__host__ __device__ inline long long ordered_bits(unsigned long long k)
+{
+    return (long long)(k >> 63 ? k & ~(1ull << 63) : ~k);
+}
+
 // ROp: explicit rows d, xm, xp, ym, yp, zm, zp (each a split field); used for
 // convection (upwind or Scharfetter-Gummel) and for transposed operators.
 template <class T>

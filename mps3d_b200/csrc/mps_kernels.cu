@@ -141,7 +141,8 @@ __global__ void k_maxabs(Lev L, const double* __restrict__ g, int rel, unsigned 
 
 // the maxima of |field| over the interior of every present field in one pass
 // (warp per row, lanes along x): out[0] vel (3 components), out[1] reac,
-// out[2] |dcoeff - dcoeff(1,1,1)|, out[3] source, out[4] soln, out[5] dcoeff;
+// out[2] |dcoeff - dcoeff(1,1,1)|, out[3] source, out[4] soln, out[5] dcoeff, the
+// coefficient's changes and the largest signed reaction (DET_WORDS);
 // NaN/Inf sort above every finite value (atomicMax on the bit patterns)
 __global__ void k_maxabs_all(Lev L, const double* __restrict__ vel, const double* __restrict__ reac,
                              const double* __restrict__ dcoeff, const double* __restrict__ source,
@@ -152,6 +153,7 @@ __global__ void k_maxabs_all(Lev L, const double* __restrict__ vel, const double
     const long long ng = gx * gy * (L.nz + 2);
     const double ref = dcoeff[1 + gx * (1 + gy)];
     long long m[6] = {0, 0, 0, 0, 0, 0};
+    unsigned long long top = 0;
     unsigned nvx = 0, nvr = 0;
     auto upd = [](long long& cur, double v) {
         v = fabs(v);
@@ -183,7 +185,10 @@ __global__ void k_maxabs_all(Lev L, const double* __restrict__ vel, const double
                 upd(m[0], vel[g + ng]);
                 upd(m[0], vel[g + 2 * ng]);
             }
-            if (reac) upd(m[1], reac[g]);
+            if (reac) {
+                upd(m[1], reac[g]);
+                top = max(top, ordered_key(__double_as_longlong(reac[g])));
+            }
             upd(m[2], d - ref);
             upd(m[5], d);
             upd(m[3], source[g]);
@@ -199,6 +204,7 @@ __global__ void k_maxabs_all(Lev L, const double* __restrict__ vel, const double
         }
         if (lane == 0 && b > 0) atomicMax(out + q, (unsigned long long)b);
     }
+    if (reac) reduce_top(top, out + DET_REAC);
     nvx = __reduce_add_sync(0xffffffffu, nvx);
     nvr = __reduce_add_sync(0xffffffffu, nvr);
     if (lane == 0 && nvx) atomicAdd(out + 6, (unsigned long long)nvx);

@@ -1934,6 +1934,12 @@ __global__ void k_unpack_nat(Lev L, CSplit<T> in, double* __restrict__ g)
 
 // max |x| over the interior of a ghosted field (x - x(1,1,1) when rel=1),
 // reduced with an integer atomicMax on the bit pattern (valid for >= 0)
+// a warp's largest ordered_key into *out
+__device__ __forceinline__ void reduce_top(unsigned long long top, unsigned long long* out)
+{
+    for (int o = 16; o > 0; o >>= 1) top = max(top, __shfl_down_sync(0xffffffffu, top, o));
+    if ((threadIdx.x & 31) == 0) atomicMax(out, top);
+}
 __global__ void k_maxabs(Lev L, const double* __restrict__ g, int rel, unsigned long long* out);
 __global__ void k_maxabs_all(Lev L, const double* __restrict__ vel, const double* __restrict__ reac,
                              const double* __restrict__ dcoeff, const double* __restrict__ source,

@@ -238,7 +238,7 @@ struct Ctx {
     bool red0_ready = false;  // the finest level's first red pass from zero was written by the outer residual
     bool redz[MAXL] = {};     // level l's first red pass from zero was written by the restriction into it
     bool sub_allowed = true;  // MPS_SUBCYCLE=0 at handle creation: one launch per pass on every level (for comparisons)
-    bool relaxed = false;     // over-relaxed passes and averaged-face coarse coefficients (solve_impl)
+    int relaxed = 0;          // levels with over-relaxed passes; with any, averaged-face coarse coefficients (solve_impl)
     size_t inbuf_bytes = 0;
     Signature sig;
     int nlev = 0;
@@ -907,10 +907,39 @@ static bool tma_prepare(int dev)
 // the colour's half in each.
 constexpr double OMEGA_FIRST = 1.6;   // the first pre-smoothing sweep
 constexpr double OMEGA_LATER = 1.4;   // the other passes of the levels below the finest
-// pre: pre-smoothing, sw: sweep, c: colour
-static double pass_omega(bool relaxed, int l, const mps_solver_opts* o, bool pre, int sw, int c)
+// Where the diagonal extra (1/dt, a sink) outweighs the faces, a plain pass is nearly
+// exact and an over-relaxed one overshoots, so a level whose extra exceeds this
+// part of its face sum keeps plain passes, and with it every coarser level (their
+// face sums fall by four).  V-cycles to 1e-11 in an FP64 CPU model, 32^3, extra over
+// the finest face sum 0.3 / 1 / 3 / 10 / 100: V(2,2) plain 5 / 4 / 3 / 2 / 1, relaxed
+// everywhere 6 / 5 / 3 / 2 / 2; V(1,1) 9 / 7 / 5 / 4 / 2 and 9 / 8 / 8 / 6 / 4.  Below
+// the line relaxing wins (V(1,1) at 0.1: 9 against 12); with the line at 0.2 no count
+// exceeds the plain one either, at 0.3 some do
+constexpr double RELAX_EXTRA = 0.15;
+// the smallest diagonal extra of a cell, from the detection's words
+static double diag_extra_min(double dtinv, double maxreac, unsigned long long top)
 {
-    if (!relaxed) return 1.0;
+    if (!(maxreac > 0.0) || !top) return dtinv;
+    const long long b = ordered_bits(top);
+    double r;
+    std::memcpy(&r, &b, sizeof(r));
+    return dtinv - r;
+}
+// how many levels from the finest over-relax, given the smallest diagonal extra and
+// the largest coefficient
+static int relaxed_levels(const Lev* lev, int nl, double extra, double maxk)
+{
+    for (int l = 0; l < nl && extra > 0.0; l++) {
+        double faces = 0.0;
+        for (int a = 0; a < 3; a++) faces += lev_n(lev[l], a) > 1 ? 2.0 * lev[l].cr[a] : 0.0;
+        if (extra > RELAX_EXTRA * maxk * faces) return l;
+    }
+    return MAXL;
+}
+// pre: pre-smoothing, sw: sweep, c: colour; relaxed: Ctx::relaxed
+static double pass_omega(int relaxed, int l, const mps_solver_opts* o, bool pre, int sw, int c)
+{
+    if (l >= relaxed) return 1.0;
     if (pre && c == 1 && sw == o->nu1 - 1) return 1.0;  // the restriction counts on a vanishing black residual
     if (pre && sw == 0) return OMEGA_FIRST;
     if (l == 0 || (!pre && sw == 0 && c == 0)) return 1.0;  // the prolongation corrects the black cells only
@@ -1336,7 +1365,7 @@ static int cl_rows(Ctx& ctx, Hier<T>& H, const Op* ops)
     return 0;
 }
 
-static double pass_omega(bool relaxed, int l, const mps_solver_opts* o, bool pre, int sw, int c);
+static double pass_omega(int relaxed, int l, const mps_solver_opts* o, bool pre, int sw, int c);
 
 // the V-cycle from level H.cl_l0 to the coarsest and back in one launch
 template <class T, class Op>
@@ -1825,8 +1854,8 @@ static int coarse_inverse(Ctx& ctx, Hier<T>& H, const Op& op)
 // prepare_only: stop after the set-up (hierarchy, operators, right-hand side,
 // initial guess, coarsest inverse), for the batched driver
 // det (optional): the operator detection of these inputs already read back
-// (k_maxabs_all's eight words, then the coefficient of cell (1,1,1)); the
-// batched solve detects every problem with one device->host read
+// (DET_WORDS words); the batched solve detects every problem with one
+// device->host read
 static int solve_impl(Ctx& ctx, const mps_grid* g, int timederiv, double dt, const Inputs& in, const int bc[6],
                       const mps_solver_opts* o, mps_solve_info* info, int ref_norm_only, int prepare_only = 0,
                       const unsigned long long* det = nullptr)
@@ -1913,13 +1942,13 @@ static int solve_impl(Ctx& ctx, const mps_grid* g, int timederiv, double dt, con
     unsigned long long* dm = ctx.dmax;
     const long long ncell = (long long)L0.nx * L0.ny * L0.nz;
     const long long ng = (long long)(L0.nx + 2) * (L0.ny + 2) * (L0.nz + 2);
-    unsigned long long hm[8];
+    unsigned long long hm[DET_WORDS];
     double k0 = 0.0;
     if (det) {
         std::memcpy(hm, det, sizeof(hm));
-        std::memcpy(&k0, det + 8, sizeof(double));
+        std::memcpy(&k0, det + DET_REF, sizeof(double));
     } else {
-        CK(cudaMemsetAsync(dm, 0, sizeof(unsigned long long) * 8, ctx.s));
+        CK(cudaMemsetAsync(dm, 0, sizeof(hm), ctx.s));
         const unsigned mb = std::min<unsigned>(nblk(ncell), 1184);
         pdl_launch(k_maxabs_all, mb, TPB, 0, ctx.s, L0, in.vel, in.reac, in.dcoeff, in.source, in.soln, dm);
         CKL();
@@ -1956,10 +1985,13 @@ static int solve_impl(Ctx& ctx, const mps_grid* g, int timederiv, double dt, con
     // The solves on the geometric hierarchy with a cell coefficient over-relax
     // their passes (pass_omega) and take the coarse coefficients of
     // k_restrict_coef; mps_vcycle_once, which is one perform_vcycle, the
-    // reference's hierarchy, explicit rows (not symmetric) and V-cycles
-    // without a relaxed first sweep or post-smoothing keep plain Gauss-Seidel
-    // and arithmetic means.
-    ctx.relaxed = sig.opclass == 0 && o->hierarchy == MPS_HIER_GEOM && !ref_norm_only && o->nu1 >= 1 && o->nu2 >= 1;
+    // reference's hierarchy, explicit rows (not symmetric), V-cycles
+    // without a relaxed first sweep or post-smoothing, and levels whose diagonal
+    // extra outweighs their faces keep plain Gauss-Seidel, and without a relaxed
+    // level arithmetic means.
+    ctx.relaxed = 0;
+    if (sig.opclass == 0 && o->hierarchy == MPS_HIER_GEOM && !ref_norm_only && o->nu1 >= 1 && o->nu2 >= 1)
+        ctx.relaxed = relaxed_levels(ctx.lev, nl, diag_extra_min(dtinv, maxreac, hm[DET_REAC]), maxk);
     // both hierarchies stay allocated (switching precision costs no allocation);
     // only the one this solve uses is filled
     int st = setup_workspace(ctx, sig, o, 1, 1);
@@ -2518,7 +2550,7 @@ int mps_create(mps_handle* h, int device)
     if (cudaStreamCreateWithFlags(&ctx.s, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreate(&ctx.e0) != cudaSuccess || cudaEventCreate(&ctx.e1) != cudaSuccess ||
         cudaMallocHost((void**)&ctx.hpin, sizeof(double) * 512) != cudaSuccess ||
-        cudaMalloc((void**)&ctx.dmax, sizeof(unsigned long long) * 8) != cudaSuccess) {
+        cudaMalloc((void**)&ctx.dmax, sizeof(unsigned long long) * DET_WORDS) != cudaSuccess) {
         delete H;
         return MPS_ERR_CUDA;
     }
