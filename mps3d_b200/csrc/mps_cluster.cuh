@@ -53,12 +53,28 @@ constexpr int CL_MAXL = 12;               // levels of one launch, the coarsest 
 constexpr int CL_TPB = 576;               // threads of a block: a column each of a 33 x 33 level, 96 registers
 constexpr int CL_GATHER = 1024;           // cells of a level that one block takes alone
 constexpr int CL_SMEM_MAX = 224 * 1024;   // shared-memory bytes of a block at most
-// cells of one colour of the top level's largest share at most, beyond which one
-// launch per pass on the whole chip is faster: uniform coefficient (65^3 in FP32,
-// 10.7 K cells: 9 us a pass against 4.5) / explicit rows, whose words come from L2
-// (64^3 in FP32, 8.2 K cells: 6.5 us against 5.5; step at 129^3 5.82 against 5.54 ms)
-constexpr int CL_MAX_SHARE = 6144;
-constexpr int CL_MAX_ROWS = 4096;
+// Cells of one colour in the largest block's share of the top level at most: beyond it
+// one launch per pass on the whole chip is faster.  Explicit rows come from L2, in FP64
+// at twice the words, and the launches for row operators (convection) read them with
+// less around it than those for a cell coefficient do, so the lines differ.  Few
+// blocks, of a level with few planes, replace launches that were small themselves.
+// us a V-cycle with the level in the cluster / with its own launches, on a B200:
+//   uniform    FP64 36^3 (2592 cells, 16 blocks) 109 / 119, 33x65x33 (3315) 131 / 122;
+//              FP32 42^3 (3528) 85 / 90, 64x64x16 (4096, 8 blocks) 103 / 89
+//   cell FP32  36^3 87 / 91; 40x33x65 104 / 95.  FP64 33^3 (1683) 111 / 121; 100x83x61
+//              (2050 at 50x41x30) 210 / 198; 150x20x10 (3000, 5 blocks) 154 / 120
+//   convection FP32 50x41x30 (2050) 81 / 87, 36^3 86 / 81; FP64 33^3 112 / 103, 64^3
+//              (1024 at 32^3) 160 / -
+//   one block  uniform FP32 64x64x1 (2048) 80 / 59, FP64 45x50x1 (1150) 81 / 84, 100x100x2
+//              (1250 at 50x50x1) 131 / 119; three blocks 48x40x6 (1920) 84 / 97
+template <class T>
+constexpr int cl_max_share(bool rows, bool row_operator, int blocks)
+{
+    const int most = sizeof(T) == 4 ? (!rows ? 3600 : row_operator ? 2200 : 2600)
+                                    : (!rows ? 3000 : row_operator ? 1100 : 1750);
+    const int few = 800 + 400 * blocks;
+    return most < few ? most : few;
+}
 
 // one fine position along one axis of a transfer: the offsets of two coarse
 // cells in the coarse ghosted layout (x, gx y, gp z; z counted from plane 0) and
@@ -111,6 +127,7 @@ struct ClPlan {
     int stage_off, part_off;     // byte offsets: restricted planes of the last split level, coarsest partial sums
     int ax_off, lin_off;         // byte offsets of the tables
     int nax, nlin, zero_vecs;    // table entries; 16-byte words of all u and f (cleared at the start)
+    int share;                   // cells of one colour in the largest block of the top level
     T kc, dexc;                  // uniform coefficient / diagonal extra
     ClLev<T> lev[CL_MAXL];
 };

@@ -1157,7 +1157,7 @@ static void cl_axes(const Lev& L, int gx, std::vector<ClAx<T>>& out)
 // the launch plan from level l0: split levels and their planes, shared-memory
 // layout, tables (ax, lin); false when it does not fit
 template <class T>
-static bool cl_layout(const Ctx& ctx, int l0, bool rows, ClPlan<T>& P, size_t& smem, std::vector<ClAx<T>>& ax,
+static bool cl_layout(const Ctx& ctx, int l0, ClPlan<T>& P, size_t& smem, std::vector<ClAx<T>>& ax,
                       std::vector<ClLin<T>>& lin)
 {
     std::memset(&P, 0, sizeof(P));
@@ -1199,7 +1199,7 @@ static bool cl_layout(const Ctx& ctx, int l0, bool rows, ClPlan<T>& P, size_t& s
             held = 0;
             for (int r = 0; r < P.nc; r++) held = std::max(held, G.z[r + 1] - G.z[r]);
         }
-        if (s == 0 && (long long)L.nh * L.ny * held > (rows ? CL_MAX_ROWS : CL_MAX_SHARE)) return false;
+        if (s == 0) P.share = L.nh * L.ny * held;
         G.uo = (int)off;
         off += (long long)G.gp * (held + 2);
         G.fo = (int)off;
@@ -1305,7 +1305,8 @@ static bool cl_setup(Ctx& ctx, Hier<T>& H, const Signature& sig)
     for (int l = 0; l < ctx.nlev; l++)
         if (odd_periodic(ctx.lev[l])) odd = l;
     for (int l = odd + 1; l < ctx.nlev - 1; l++) {
-        if (!cl_layout<T>(ctx, l, rows, *P, smem, ax, lin)) continue;
+        if (!cl_layout<T>(ctx, l, *P, smem, ax, lin) || P->share > cl_max_share<T>(rows, sig.opclass == 1, P->nc))
+            continue;
         H.cl_l0 = l;
         break;
     }
@@ -1331,7 +1332,7 @@ static int cl_tables(Ctx& ctx, Hier<T>& H)
     std::vector<ClAx<T>> ax;
     std::vector<ClLin<T>> lin;
     size_t smem = 0;
-    if (!cl_layout<T>(ctx, H.cl_l0, H.crow[H.cl_l0] != nullptr, *P, smem, ax, lin)) {
+    if (!cl_layout<T>(ctx, H.cl_l0, *P, smem, ax, lin)) {
         ctx.err.msg = "cluster plan";
         return MPS_ERR_CUDA;
     }
@@ -1378,7 +1379,7 @@ static int cluster_cycle(Ctx& ctx, Hier<T>& H, const Op* ops, const mps_solver_o
     std::vector<ClLin<T>> lin;
     size_t smem = 0;
     const bool rows = H.crow[l0] != nullptr;
-    if (!cl_layout<T>(ctx, l0, rows, P, smem, ax, lin)) {
+    if (!cl_layout<T>(ctx, l0, P, smem, ax, lin)) {
         ctx.err.msg = "cluster plan";
         return MPS_ERR_CUDA;
     }
