@@ -820,7 +820,7 @@ static void plan_batch(BatchState& B, BatchPlan<T>& P, const mps_solver_opts* o,
                 x.u1 = cur1(p, d);
                 x.out = c == 0 ? H.U[d][ri[p][d] ^ 1] : H.U[d][bi[p][d] ^ 1] + L.half;
                 x.f = H.F[d] + (c ? L.half : 0);
-                x.om = (T)pass_omega(sc.relaxed, d, o, pre, sw, c);
+                x.om = (T)pass_omega(sc, d, o, pre, sw, c);
                 x.split = batch_vector_level(L) && make_split(L, BATCH_W, x.cs) ? 1 : 0;
                 if (!x.split) std::memset(&x.cs, 0, sizeof(x.cs));
                 if (c == 0) ri[p][d] ^= 1;
@@ -1137,18 +1137,12 @@ static std::vector<long long> prep_key_of(int wordsize, int np, const mps_proble
             long long kb = 0;
             if (kuni) std::memcpy(&kb, &v[DET_REF], 8);  // the uniform coefficient enters the operators
             k.push_back(kb);
-            // the levels with over-relaxed passes
+            // the weight of the diagonal extra (the passes' relaxation)
             const mps_problem& q = probs[p];
-            const double dmin = diag_extra_min(q.timederiv && q.dt > 0 ? 1.0 / q.dt : 0.0, v[1],
-                                               det[(size_t)DET_WORDS * p + DET_REAC]);
-            int nrel = MAXL;
-            if (dmin > 0 && o->hierarchy == MPS_HIER_GEOM) {
-                Lev lev[MAXL];
-                Xfer xf[MAXL];
-                std::string why;
-                nrel = relaxed_levels(lev, plan_levels(&q.g, o, q.bc_code, lev, xf, why), dmin, v[5]);
-            }
-            k.push_back(nrel);
+            const double extra = diag_extra_min(q.timederiv && q.dt > 0 ? 1.0 / q.dt : 0.0, v[1],
+                                                det[(size_t)DET_WORDS * p + DET_REAC]);
+            const double llen[3] = {q.g.llenx, q.g.lleny, q.g.llenz};
+            k.push_back(extra_step(make_lev_uniform(q.g.lx, q.g.ly, q.g.lz, llen, q.bc_code), extra, v[5]));
         }
     }
     return k;

@@ -141,8 +141,8 @@ __global__ void k_maxabs(Lev L, const double* __restrict__ g, int rel, unsigned 
 
 // the maxima of |field| over the interior of every present field in one pass
 // (warp per row, lanes along x): out[0] vel (3 components), out[1] reac,
-// out[2] |dcoeff - dcoeff(1,1,1)|, out[3] source, out[4] soln, out[5] dcoeff, the
-// coefficient's changes and the largest signed reaction (DET_WORDS);
+// out[2] |dcoeff - dcoeff(1,1,1)|, out[3] source, out[4] soln, out[5] dcoeff, and
+// the coefficient's changes (DET_WORDS);
 // NaN/Inf sort above every finite value (atomicMax on the bit patterns)
 __global__ void k_maxabs_all(Lev L, const double* __restrict__ vel, const double* __restrict__ reac,
                              const double* __restrict__ dcoeff, const double* __restrict__ source,
@@ -153,7 +153,6 @@ __global__ void k_maxabs_all(Lev L, const double* __restrict__ vel, const double
     const long long ng = gx * gy * (L.nz + 2);
     const double ref = dcoeff[1 + gx * (1 + gy)];
     long long m[6] = {0, 0, 0, 0, 0, 0};
-    unsigned long long top = 0;
     unsigned nvx = 0, nvr = 0;
     auto upd = [](long long& cur, double v) {
         v = fabs(v);
@@ -185,10 +184,7 @@ __global__ void k_maxabs_all(Lev L, const double* __restrict__ vel, const double
                 upd(m[0], vel[g + ng]);
                 upd(m[0], vel[g + 2 * ng]);
             }
-            if (reac) {
-                upd(m[1], reac[g]);
-                top = max(top, ordered_key(__double_as_longlong(reac[g])));
-            }
+            if (reac) upd(m[1], reac[g]);
             upd(m[2], d - ref);
             upd(m[5], d);
             upd(m[3], source[g]);
@@ -204,11 +200,27 @@ __global__ void k_maxabs_all(Lev L, const double* __restrict__ vel, const double
         }
         if (lane == 0 && b > 0) atomicMax(out + q, (unsigned long long)b);
     }
-    if (reac) reduce_top(top, out + DET_REAC);
     nvx = __reduce_add_sync(0xffffffffu, nvx);
     nvr = __reduce_add_sync(0xffffffffu, nvr);
     if (lane == 0 && nvx) atomicAdd(out + 6, (unsigned long long)nvx);
     if (lane == 0 && nvr) atomicAdd(out + 7, (unsigned long long)nvr);
+}
+
+// the largest signed reaction, for operators that have one (in k_maxabs_all its
+// registers cost every solve 25 us of the scan's 100 at 257^3)
+__global__ void k_max_reac(Lev L, const double* __restrict__ reac, unsigned long long* out)
+{
+    pdl_wait();
+    const long long gx = L.nx + 2, gy = L.ny + 2;
+    unsigned long long top = 0;
+    const unsigned lane = threadIdx.x & 31;
+    const unsigned warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarp = (gridDim.x * blockDim.x) >> 5;
+    for (unsigned row = warp; row < L.rows; row += nwarp) {
+        const unsigned k = L.divNy.div(row), j = row - k * (unsigned)L.ny;
+        const double* r = reac + 1 + gx * ((long long)(j + 1) + gy * (long long)(k + 1));
+        for (int i = lane; i < L.nx; i += 32) top = max(top, ordered_key(__double_as_longlong(r[i])));
+    }
+    reduce_top(top, out);
 }
 
 __global__ void k_fill_ghosts(Lev L, double* __restrict__ g, const double* bl, const double* br, const double* bb,

@@ -1940,6 +1940,7 @@ __device__ __forceinline__ void reduce_top(unsigned long long top, unsigned long
     for (int o = 16; o > 0; o >>= 1) top = max(top, __shfl_down_sync(0xffffffffu, top, o));
     if ((threadIdx.x & 31) == 0) atomicMax(out, top);
 }
+__global__ void k_max_reac(Lev L, const double* __restrict__ reac, unsigned long long* out);
 __global__ void k_maxabs(Lev L, const double* __restrict__ g, int rel, unsigned long long* out);
 __global__ void k_maxabs_all(Lev L, const double* __restrict__ vel, const double* __restrict__ reac,
                              const double* __restrict__ dcoeff, const double* __restrict__ source,

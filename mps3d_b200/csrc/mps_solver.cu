@@ -189,13 +189,13 @@ struct Prof {
 // that is baked into its kernel parameters
 struct GraphKey {
     Signature sig;
-    int kind = -1, prec = -1, inner = 0, nu1 = 0, nu2 = 0, nlev = 0, flux = 0, transpose = 0, prof = 0, relaxed = 0, kseg = 0;
+    int kind = -1, prec = -1, inner = 0, nu1 = 0, nu2 = 0, nlev = 0, flux = 0, transpose = 0, prof = 0, relaxed = 0, extra_q = 0, kseg = 0;
     double kc = 0, dexc = 0;
     double len[3] = {0, 0, 0};  // the box: the levels' face coefficients
     const void* ws = nullptr;  // workspace identity (first arena block)
     bool operator==(const GraphKey& o) const
     {
-        return sig == o.sig && std::equal(len, len + 3, o.len) && relaxed == o.relaxed && kseg == o.kseg && kind == o.kind && prec == o.prec && inner == o.inner && nu1 == o.nu1 &&
+        return sig == o.sig && std::equal(len, len + 3, o.len) && relaxed == o.relaxed && extra_q == o.extra_q && kseg == o.kseg && kind == o.kind && prec == o.prec && inner == o.inner && nu1 == o.nu1 &&
                nu2 == o.nu2 && nlev == o.nlev && flux == o.flux && transpose == o.transpose && prof == o.prof &&
                kc == o.kc &&
                dexc == o.dexc && ws == o.ws;
@@ -238,7 +238,9 @@ struct Ctx {
     bool red0_ready = false;  // the finest level's first red pass from zero was written by the outer residual
     bool redz[MAXL] = {};     // level l's first red pass from zero was written by the restriction into it
     bool sub_allowed = true;  // MPS_SUBCYCLE=0 at handle creation: one launch per pass on every level (for comparisons)
-    int relaxed = 0;          // levels with over-relaxed passes; with any, averaged-face coarse coefficients (solve_impl)
+    bool relaxed = false;     // over-relaxed passes and averaged-face coarse coefficients (solve_impl)
+    int extra_q = 0;          // the diagonal extra's weight (extra_step), and with it
+    double relax[MAXL] = {};  // the part of the over-relaxation that each level takes
     size_t inbuf_bytes = 0;
     Signature sig;
     int nlev = 0;
@@ -908,14 +910,15 @@ static bool tma_prepare(int dev)
 constexpr double OMEGA_FIRST = 1.6;   // the first pre-smoothing sweep
 constexpr double OMEGA_LATER = 1.4;   // the other passes of the levels below the finest
 // Where the diagonal extra (1/dt, a sink) outweighs the faces, a plain pass is nearly
-// exact and an over-relaxed one overshoots, so a level whose extra exceeds this
-// part of its face sum keeps plain passes, and with it every coarser level (their
-// face sums fall by four).  V-cycles to 1e-11 in an FP64 CPU model, 32^3, extra over
-// the finest face sum 0.3 / 1 / 3 / 10 / 100: V(2,2) plain 5 / 4 / 3 / 2 / 1, relaxed
-// everywhere 6 / 5 / 3 / 2 / 2; V(1,1) 9 / 7 / 5 / 4 / 2 and 9 / 8 / 8 / 6 / 4.  Below
-// the line relaxing wins (V(1,1) at 0.1: 9 against 12); with the line at 0.2 no count
-// exceeds the plain one either, at 0.3 some do
-constexpr double RELAX_EXTRA = 0.15;
+// exact and an over-relaxed one overshoots.  So a level relaxes by 1 + (w - 1) / (1 + r)^2,
+// r its smallest diagonal extra over its face sum (which falls by four from level to
+// level), and plainly where less than RELAX_LEAST is left.  V-cycles to 1e-11 in an FP64
+// CPU model, 32^3, extra over the finest face sum 0.1 / 0.3 / 1 / 3 / 10 / 100, plain ->
+// relaxed alike on every level -> this: V(2,2) 7 / 5 / 4 / 3 / 2 / 1 -> 7 / 6 / 5 / 3 / 2 / 2 ->
+// 6 / 5 / 3 / 2 / 2 / 1, V(1,1) 12 / 9 / 7 / 5 / 4 / 2 -> 9 / 9 / 8 / 8 / 6 / 4 ->
+// 8 / 7 / 6 / 4 / 3 / 2.  Of the powers of 1 / (1 + r), 2 is the lowest that took no more cycles
+// than plain passes anywhere (1.5 to 4, V(1,1) to V(3,3), three boxes, r to 1000)
+constexpr double RELAX_LEAST = 0.02;
 // the smallest diagonal extra of a cell, from the detection's words
 static double diag_extra_min(double dtinv, double maxreac, unsigned long long top)
 {
@@ -925,25 +928,41 @@ static double diag_extra_min(double dtinv, double maxreac, unsigned long long to
     std::memcpy(&r, &b, sizeof(r));
     return dtinv - r;
 }
-// how many levels from the finest over-relax, given the smallest diagonal extra and
-// the largest coefficient
-static int relaxed_levels(const Lev* lev, int nl, double extra, double maxk)
+// the diagonal extra over the finest face sum in half powers of two: what the
+// relaxation depends on, and a captured launch sequence with it, must not change with
+// every digit of a reaction field.  EXTRA_NONE: none that a level would feel
+constexpr int EXTRA_NONE = -1000;
+static double face_sum(const Lev& L)
 {
-    for (int l = 0; l < nl && extra > 0.0; l++) {
-        double faces = 0.0;
-        for (int a = 0; a < 3; a++) faces += lev_n(lev[l], a) > 1 ? 2.0 * lev[l].cr[a] : 0.0;
-        if (extra > RELAX_EXTRA * maxk * faces) return l;
-    }
-    return MAXL;
+    double s = 0.0;
+    for (int a = 0; a < 3; a++) s += lev_n(L, a) > 1 ? 2.0 * L.cr[a] : 0.0;
+    return s;
 }
-// pre: pre-smoothing, sw: sweep, c: colour; relaxed: Ctx::relaxed
-static double pass_omega(int relaxed, int l, const mps_solver_opts* o, bool pre, int sw, int c)
+static int extra_step(const Lev& L0, double extra, double maxk)
 {
-    if (l >= relaxed) return 1.0;
+    if (!(extra > 1e-6 * maxk * face_sum(L0))) return EXTRA_NONE;
+    return (int)std::lround(2.0 * std::log2(std::min(extra / std::max(maxk * face_sum(L0), 1e-300), 1e6)));
+}
+// Ctx::relax of every level; without a level that relaxes, Ctx::relaxed goes
+static void set_relaxation(Ctx& ctx)
+{
+    const double r0 = ctx.extra_q == EXTRA_NONE ? 0.0 : std::exp2(0.5 * ctx.extra_q), f0 = face_sum(ctx.lev[0]);
+    for (int l = 0; l < ctx.nlev; l++) {
+        const double f = face_sum(ctx.lev[l]), r = f > 0.0 ? r0 * f0 / f : r0;
+        ctx.relax[l] = 1.0 / ((1.0 + r) * (1.0 + r));
+    }
+    ctx.relaxed = ctx.relaxed && (OMEGA_FIRST - 1.0) * ctx.relax[0] >= RELAX_LEAST;
+}
+// pre: pre-smoothing, sw: sweep, c: colour
+static double pass_omega(const Ctx& ctx, int l, const mps_solver_opts* o, bool pre, int sw, int c)
+{
+    if (!ctx.relaxed) return 1.0;
     if (pre && c == 1 && sw == o->nu1 - 1) return 1.0;  // the restriction counts on a vanishing black residual
-    if (pre && sw == 0) return OMEGA_FIRST;
-    if (l == 0 || (!pre && sw == 0 && c == 0)) return 1.0;  // the prolongation corrects the black cells only
-    return OMEGA_LATER;
+    double w = OMEGA_LATER;
+    if (pre && sw == 0) w = OMEGA_FIRST;
+    else if (l == 0 || (!pre && sw == 0 && c == 0)) return 1.0;  // the prolongation corrects the black cells only
+    const double excess = (w - 1.0) * ctx.relax[l];
+    return excess < RELAX_LEAST ? 1.0 : 1.0 + excess;
 }
 
 // ---- one colour pass ----
@@ -1366,7 +1385,7 @@ static int cl_rows(Ctx& ctx, Hier<T>& H, const Op* ops)
     return 0;
 }
 
-static double pass_omega(int relaxed, int l, const mps_solver_opts* o, bool pre, int sw, int c);
+static double pass_omega(const Ctx& ctx, int l, const mps_solver_opts* o, bool pre, int sw, int c);
 
 // the V-cycle from level H.cl_l0 to the coarsest and back in one launch
 template <class T, class Op>
@@ -1389,8 +1408,8 @@ static int cluster_cycle(Ctx& ctx, Hier<T>& H, const Op* ops, const mps_solver_o
     P.load_u = !zero_guess;
     for (int s = 0; s < P.nl; s++) {
         const int l = l0 + s;
-        P.lev[s].om0 = (T)pass_omega(ctx.relaxed, l, o, true, 0, 0);
-        P.lev[s].om1 = (T)pass_omega(ctx.relaxed, l, o, false, 0, 1);
+        P.lev[s].om0 = (T)pass_omega(ctx, l, o, true, 0, 0);
+        P.lev[s].om1 = (T)pass_omega(ctx, l, o, false, 0, 1);
         P.lev[s].half = ctx.lev[l].half;
         P.lev[s].rows = H.crow[l];
     }
@@ -1431,7 +1450,7 @@ static int vcycle_rec(Ctx& ctx, Hier<T>& H, const Op* ops, int l, const mps_solv
     const Lev& L = ctx.lev[l];
     const Lev& C = ctx.lev[l + 1];
     int st;
-    auto om = [&](bool pre, int sw, int c) { return pass_omega(ctx.relaxed, l, o, pre, sw, c); };
+    auto om = [&](bool pre, int sw, int c) { return pass_omega(ctx, l, o, pre, sw, c); };
     for (int s = 0; s < o->nu1; s++) {
         bool z = zero_guess && s == 0;
         if (z && ((l == 0 && ctx.red0_ready) || ctx.redz[l])) {
@@ -1953,6 +1972,10 @@ static int solve_impl(Ctx& ctx, const mps_grid* g, int timederiv, double dt, con
         const unsigned mb = std::min<unsigned>(nblk(ncell), 1184);
         pdl_launch(k_maxabs_all, mb, TPB, 0, ctx.s, L0, in.vel, in.reac, in.dcoeff, in.source, in.soln, dm);
         CKL();
+        if (in.reac) {
+            pdl_launch(k_max_reac, mb, TPB, 0, ctx.s, L0, in.reac, dm + DET_REAC);
+            CKL();
+        }
         CK(cudaMemcpyAsync(hm, dm, sizeof(hm), cudaMemcpyDeviceToHost, ctx.s));
         CK(cudaMemcpyAsync(&k0, in.dcoeff + 1 + (L0.nx + 2) * (1 + (long long)(L0.ny + 2)), sizeof(double),
                            cudaMemcpyDeviceToHost, ctx.s));
@@ -1986,13 +2009,12 @@ static int solve_impl(Ctx& ctx, const mps_grid* g, int timederiv, double dt, con
     // The solves on the geometric hierarchy with a cell coefficient over-relax
     // their passes (pass_omega) and take the coarse coefficients of
     // k_restrict_coef; mps_vcycle_once, which is one perform_vcycle, the
-    // reference's hierarchy, explicit rows (not symmetric), V-cycles
-    // without a relaxed first sweep or post-smoothing, and levels whose diagonal
-    // extra outweighs their faces keep plain Gauss-Seidel, and without a relaxed
-    // level arithmetic means.
-    ctx.relaxed = 0;
-    if (sig.opclass == 0 && o->hierarchy == MPS_HIER_GEOM && !ref_norm_only && o->nu1 >= 1 && o->nu2 >= 1)
-        ctx.relaxed = relaxed_levels(ctx.lev, nl, diag_extra_min(dtinv, maxreac, hm[DET_REAC]), maxk);
+    // reference's hierarchy, explicit rows (not symmetric) and V-cycles
+    // without a relaxed first sweep or post-smoothing keep plain Gauss-Seidel
+    // and arithmetic means.
+    ctx.relaxed = sig.opclass == 0 && o->hierarchy == MPS_HIER_GEOM && !ref_norm_only && o->nu1 >= 1 && o->nu2 >= 1;
+    ctx.extra_q = extra_step(L0, diag_extra_min(dtinv, maxreac, hm[DET_REAC]), maxk);
+    set_relaxation(ctx);
     // both hierarchies stay allocated (switching precision costs no allocation);
     // only the one this solve uses is filled
     int st = setup_workspace(ctx, sig, o, 1, 1);
@@ -2155,7 +2177,7 @@ static int solve_impl(Ctx& ctx, const mps_grid* g, int timederiv, double dt, con
                 if (!H.D[l]) continue;
                 const Lev& Ll = ctx.lev[l];
                 pdl_launch(k_diag_red<TT, KOp<TT>>, nblk((long long)Ll.P * Ll.rows), TPB, 0, ctx.s, Ll, H.kop[l],
-                           H.D[l], (TT)pass_omega(ctx.relaxed, l, o, true, 0, 0));
+                           H.D[l], (TT)pass_omega(ctx, l, o, true, 0, 0));
                 CKL();
             }
             return 0;
@@ -2196,6 +2218,7 @@ static int solve_impl(Ctx& ctx, const mps_grid* g, int timederiv, double dt, con
     std::copy(ctx.len, ctx.len + 3, gk.len);
     gk.ws = ctx.ar.blocks.empty() ? nullptr : ctx.ar.blocks[0];
     gk.relaxed = ctx.relaxed;
+    gk.extra_q = ctx.relaxed ? ctx.extra_q : 0;
     gk.kseg = sig.opclass == 0 && ctx.kseg;
     gk.prof = ctx.prof.on ? 1 + ctx.prof.level : 0;  // profiled graphs carry event-record nodes
     // graphs need the buffer parities to return after one iteration
@@ -2261,7 +2284,7 @@ static int solve_impl(Ctx& ctx, const mps_grid* g, int timederiv, double dt, con
             float* ured = o->nu1 >= 1 && H.cl_l0 != 0 ? H.U[0][H.ri[0] ^ 1] : nullptr;
             if (sig.opclass == 0)
                 return resid_norm(ctx, ctx.kop64, csplit<double>(ctx.x64, L), csplit<double>(ctx.b64, L), r32, ured,
-                                  &red_ready, pass_omega(ctx.relaxed, 0, o, true, 0, 0));
+                                  &red_ready, pass_omega(ctx, 0, o, true, 0, 0));
             return resid_norm(ctx, ctx.rop64, csplit<double>(ctx.x64, L), csplit<double>(ctx.b64, L), r32, ured,
                               &red_ready);
         };
