@@ -1308,13 +1308,13 @@ static bool cl_layout(const Ctx& ctx, int l0, ClPlan<T>& P, size_t& smem, std::v
 // cl_l0 -1: none (odd periodic sizes: cells of one colour touch, and in-place
 // passes would read new values)
 template <class T>
-static bool cl_setup(Ctx& ctx, Hier<T>& H, const Signature& sig)
+static bool cl_setup(Ctx& ctx, Hier<T>& H, const Signature& sig, bool lean)
 {
     H.cl_l0 = -1;
     H.cltab = nullptr;
     H.cl_len[0] = H.cl_len[1] = H.cl_len[2] = 0.0;
     for (int l = 0; l < MAXL; l++) H.crow[l] = nullptr;
-    if (!ctx.sub_allowed || !cl_prepare(ctx.dev)) return true;
+    if (lean || !ctx.sub_allowed || !cl_prepare(ctx.dev)) return true;
     std::unique_ptr<ClPlan<T>> P(new ClPlan<T>);
     std::vector<ClAx<T>> ax;
     std::vector<ClLin<T>> lin;
@@ -1693,29 +1693,29 @@ static void alloc_hier(Ctx& ctx, Hier<T>& H, bool& ok)
 constexpr long long SEG_MIN_CELLS = 1 << 19;
 static bool seg_level(const Lev& L) { return (long long)L.nx * L.ny * L.nz >= SEG_MIN_CELLS && L.nx >= 32; }
 
-static int setup_workspace(Ctx& ctx, const Signature& sig, const mps_solver_opts* o, int need64, int need32)
+// the arrays of one signature; lean: only what a solve cannot do without -- no averaged-
+// face coarse coefficients and their means, no uniform segments, no cluster (its rows
+// are eight words a cell), the transposed rows' scratch per solve
+static bool alloc_workspace(Ctx& ctx, const Signature& sig, int need64, int need32, bool lean)
 {
-    if (sig == ctx.sig) return 0;
-    destroy_graphs(ctx);
-    ctx.ar.clear();
-    ctx.sig = Signature();
     bool ok = true;
     const int nl = ctx.nlev;
     for (int l = 0; l < nl; l++) {
         const Lev& L = ctx.lev[l];
         const size_t b64 = sizeof(double) * 2 * L.half, b32 = sizeof(float) * 2 * L.half;
         ctx.pk[l] = (double*)ctx.ar.get(b64);
-        ctx.pka[l] = (sig.opclass == 0 && !sig.kuni && l >= 1) ? (double*)ctx.ar.get(b64) : nullptr;
+        const bool means = !lean && sig.opclass == 0 && !sig.kuni && l >= 1;
+        ctx.pka[l] = means ? (double*)ctx.ar.get(b64) : nullptr;
         ctx.preac[l] = sig.has_reac ? (double*)ctx.ar.get(b64) : nullptr;
         ctx.dex64[l] = sig.has_reac ? (double*)ctx.ar.get(b64) : nullptr;
         for (int a = 0; a < 3; a++) ctx.pv[a][l] = sig.opclass == 1 ? (double*)ctx.ar.get(b64) : nullptr;
-        ok = ok && ctx.pk[l] && (ctx.pka[l] || sig.opclass != 0 || sig.kuni || l < 1);
+        ok = ok && ctx.pk[l] && (ctx.pka[l] || !means);
         if (sig.opclass == 1) {
             ctx.rows64[l] = (need64 || l == 0) ? (double*)ctx.ar.get(7 * b64) : nullptr;  // l>0: FP64 solves
             ctx.rows32[l] = need32 ? (float*)ctx.ar.get(7 * b32) : nullptr;
         } else {
             ctx.k32[l] = (need32 && !sig.kuni) ? (float*)ctx.ar.get(b32) : nullptr;
-            const bool segs = !sig.kuni && seg_level(L);
+            const bool segs = !lean && !sig.kuni && seg_level(L);
             const size_t ns = (size_t)L.rows * ((L.nh + 15) / 16);
             ctx.seg64[l] = segs ? (double*)ctx.ar.get(sizeof(double) * ns) : nullptr;
             ctx.seg32[l] = segs ? (float*)ctx.ar.get(sizeof(float) * ns) : nullptr;
@@ -1724,8 +1724,9 @@ static int setup_workspace(Ctx& ctx, const Signature& sig, const mps_solver_opts
         }
     }
     // (allocating it in every solve cost 17.1 against 14.1 ms for the 65^3 gradient)
-    ctx.trows = sig.transpose ? (double*)ctx.ar.get(sizeof(double) * 7 * 2 * ctx.lev[0].half) : nullptr;
-    ok = ok && (ctx.trows || !sig.transpose);
+    const bool trows = !lean && sig.transpose;
+    ctx.trows = trows ? (double*)ctx.ar.get(sizeof(double) * 7 * 2 * ctx.lev[0].half) : nullptr;
+    ok = ok && (ctx.trows || !trows);
     if (need64) alloc_hier(ctx, ctx.h64, ok);
     if (need32) alloc_hier(ctx, ctx.h32, ok);
     const Lev& L0 = ctx.lev[0];
@@ -1743,9 +1744,25 @@ static int setup_workspace(Ctx& ctx, const Signature& sig, const mps_solver_opts
     ok = ok && ctx.x64 && ctx.b64 && ctx.dense && ctx.gjM && ctx.dstatus && ctx.rb.partial && ctx.rb.counter &&
          ctx.rb.out;
     // the small levels in one cluster
-    if (need64) ok = ok && cl_setup<double>(ctx, ctx.h64, sig);
-    if (need32) ok = ok && cl_setup<float>(ctx, ctx.h32, sig);
+    if (need64) ok = ok && cl_setup<double>(ctx, ctx.h64, sig, lean);
+    if (need32) ok = ok && cl_setup<float>(ctx, ctx.h32, sig, lean);
+    return ok;
+}
+
+static int setup_workspace(Ctx& ctx, const Signature& sig, int need64, int need32)
+{
+    if (sig == ctx.sig) return 0;
+    destroy_graphs(ctx);
+    ctx.ar.clear();
+    ctx.sig = Signature();
+    bool ok = alloc_workspace(ctx, sig, need64, need32, false);
+    if (!ok) {  // past the cap, or the device is full: without the arrays that only buy time
+        cudaGetLastError();
+        ctx.ar.clear();
+        ok = alloc_workspace(ctx, sig, need64, need32, true);
+    }
     if (!ok) {
+        cudaGetLastError();
         ctx.ar.clear();
         ctx.err.code = MPS_ERR_NOMEM;
         ctx.err.msg = "device allocation failed";
@@ -2006,20 +2023,21 @@ static int solve_impl(Ctx& ctx, const mps_grid* g, int timederiv, double dt, con
     sig.kuni = dkvar == 0.0;
     sig.transpose = o->transpose && sig.opclass == 1;
     const bool mixed = o->precision == MPS_PREC_MIXED;
+    // both hierarchies stay allocated (switching precision costs no allocation);
+    // only the one this solve uses is filled
+    int st = setup_workspace(ctx, sig, 1, 1);
+    const int need64 = !mixed, need32 = mixed;
+    if (st) return st;
     // The solves on the geometric hierarchy with a cell coefficient over-relax
     // their passes (pass_omega) and take the coarse coefficients of
     // k_restrict_coef; mps_vcycle_once, which is one perform_vcycle, the
     // reference's hierarchy, explicit rows (not symmetric) and V-cycles
     // without a relaxed first sweep or post-smoothing keep plain Gauss-Seidel
-    // and arithmetic means.
-    ctx.relaxed = sig.opclass == 0 && o->hierarchy == MPS_HIER_GEOM && !ref_norm_only && o->nu1 >= 1 && o->nu2 >= 1;
+    // and arithmetic means, and so does a workspace without room for both means.
+    ctx.relaxed = sig.opclass == 0 && o->hierarchy == MPS_HIER_GEOM && !ref_norm_only && o->nu1 >= 1 && o->nu2 >= 1 &&
+                  (sig.kuni || nl < 2 || ctx.pka[1]);
     ctx.extra_q = extra_step(L0, diag_extra_min(dtinv, maxreac, hm[DET_REAC]), maxk);
     set_relaxation(ctx);
-    // both hierarchies stay allocated (switching precision costs no allocation);
-    // only the one this solve uses is filled
-    int st = setup_workspace(ctx, sig, o, 1, 1);
-    const int need64 = !mixed, need32 = mixed;
-    if (st) return st;
     if (o->krylov == MPS_KRYLOV_FGMRES && (st = setup_krylov(ctx, 2 * ctx.lev[0].half, o->restart))) return st;
 
     // ---- coefficient pyramid (FP64) ----
@@ -2093,7 +2111,7 @@ static int solve_impl(Ctx& ctx, const mps_grid* g, int timederiv, double dt, con
         // (four a row) from row to row (the passes then read one word for 32 cells;
         // where most segments differ, that word is one more)
         const unsigned long long nchunk = (unsigned long long)L0.rows * (unsigned)((L0.nx + 31) / 32);
-        ctx.kseg = !prepare_only && !sig.kuni && !in.vel && hm[6] <= nchunk / 4 && hm[7] <= (unsigned long long)L0.rows;
+        ctx.kseg = !prepare_only && !sig.kuni && ctx.seg64[0] && !in.vel && hm[6] <= nchunk / 4 && hm[7] <= (unsigned long long)L0.rows;
         if (ctx.kseg) {
             auto segments = [&](auto* k, auto* seg, auto& op, int l) -> int {
                 using TT = typename std::remove_pointer<decltype(seg)>::type;
@@ -2113,10 +2131,15 @@ static int solve_impl(Ctx& ctx, const mps_grid* g, int timederiv, double dt, con
         ctx.kop64 = k64[0];
         if (need64) std::copy(k64, k64 + nl, ctx.h64.kop);
     } else {
+        double* trows = ctx.trows;
+        if (sig.transpose && !trows) CK(cudaMallocAsync((void**)&trows, sizeof(double) * 7 * 2 * L0.half, ctx.s));
+        auto release = [&]() { if (trows != ctx.trows) cudaFreeAsync(trows, ctx.s); };
         for (int l = 0; l < nl; l++) {
             if (ctx.rows64[l] && (need64 || l == 0)) {
-                if ((st = build_rows_level<double>(ctx, l, ctx.rows64[l], dtinv, o->flux, sig.transpose, ctx.trows)))
+                if ((st = build_rows_level<double>(ctx, l, ctx.rows64[l], dtinv, o->flux, sig.transpose, trows))) {
+                    release();
                     return st;
+                }
                 if (need64) ctx.h64.rop[l] = make_rop<double>(ctx.rows64[l], ctx.lev[l]);
             }
             if (ctx.rows32[l] && need32) {
@@ -2129,12 +2152,14 @@ static int solve_impl(Ctx& ctx, const mps_grid* g, int timederiv, double dt, con
                                ctx.rows64[l], ctx.rows32[l], 1.0, 0.0);
                     CKL();
                 } else if ((st = build_rows_level<float>(ctx, l, ctx.rows32[l], dtinv, o->flux, sig.transpose,
-                                                         (float*)ctx.trows))) {
+                                                         (float*)trows))) {
+                    release();
                     return st;
                 }
                 ctx.h32.rop[l] = make_rop<float>(ctx.rows32[l], ctx.lev[l]);
             }
         }
+        release();
         ctx.rop64 = make_rop<double>(ctx.rows64[0], L0);
     }
     // ---- right-hand side and initial guess ----
