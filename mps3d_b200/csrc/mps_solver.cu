@@ -160,7 +160,7 @@ struct Hier {
     unsigned char* cltab = nullptr;   // its axis and interpolation tables
     std::vector<unsigned char> climg; // the host copy of the tables on the device (cl_tables)
     double cl_len[3] = {0, 0, 0};     // the box that they hold
-    T* crow[MAXL] = {};               // explicit rows of a cell coefficient on its levels (k_krows)
+    T* crow[MAXL] = {};               // explicit rows on its levels, eight words a cell (k_crows)
     double* Dprev = nullptr;  // the coarsest matrix whose inverse AinvT holds
     int* gj = nullptr;        // its inversion state (k_gauss_jordan)
 };
@@ -743,9 +743,9 @@ static RestrictSplit make_restrict_split(const Lev& F, const Lev& C, const Box& 
 // Without one (uniform, or uniform along most segments; 257^3 Poisson / plasma,
 // ms): 6 rows at 3, 4, 5 blocks - / 10.73, 5.39 / 10.37, - / 10.56; 7 rows at 4
 // blocks 5.48 / 10.86, 8 rows at 4 blocks 5.13 / 10.40
-template <class T, bool KF>
+template <bool KF>
 struct TmaShape {  // rows per block, one warp each; blocks per SM the tiling aims at; cells per thread
-    static constexpr int TJ = sizeof(T) == 8 ? 4 : (KF ? 6 : 8);
+    static constexpr int TJ = KF ? 6 : 8;
     static constexpr int BPS = KF ? 3 : 4;
     static constexpr int W = 4;
 };
@@ -774,53 +774,52 @@ static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder()
 
 // 3-D map of one colour half (P x ny x nz elements) with boxes of `rows`
 // full rows of one plane
-template <class T>
-static bool encode_half(CUtensorMap* m, const T* base, const Lev& L, int rows)
+static bool encode_half(CUtensorMap* m, const float* base, const Lev& L, int rows)
 {
     auto fn = tensor_map_encoder();
     if (!fn) return false;
     const cuuint64_t dims[3] = {(cuuint64_t)L.P, (cuuint64_t)L.ny, (cuuint64_t)L.nz};
-    const cuuint64_t strides[2] = {(cuuint64_t)L.P * sizeof(T), (cuuint64_t)L.P * L.ny * sizeof(T)};
+    const cuuint64_t strides[2] = {(cuuint64_t)L.P * sizeof(float), (cuuint64_t)L.P * L.ny * sizeof(float)};
     const cuuint32_t box[3] = {(cuuint32_t)L.P, (cuuint32_t)rows, 1};
     const cuuint32_t es[3] = {1, 1, 1};
-    return fn(m, sizeof(T) == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3,
-              const_cast<T*>(base), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    return fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float*>(base), dims, strides, box, es,
+              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// the finest level's colour pass from a valid state with k_colour_tma;
+// the finest level's FP32 colour pass from a valid state with k_colour_tma (the
+// FP64 pass measured slower through shared memory, 104-117 against 87 us at 257^3,
+// the FP32 pass faster, 49.6 against 51.2 us, both with a staged coefficient);
 // returns 1 when the pass was launched, 0 when this level or operator does
 // not qualify (the caller runs the register-fed pass), < 0 on an error
-template <class T, bool KF>
-static int colour_pass_tma_kf(Ctx& ctx, Hier<T>& H, const KOp<T>& op, int l, int c, T* out, const T* fh, T om)
+template <bool KF>
+static int colour_pass_tma_kf(Ctx& ctx, Hier<float>& H, const KOp<float>& op, int l, int c, float* out,
+                              const float* fh, float om)
 {
-    constexpr int TJ = TmaShape<T, KF>::TJ, W = TmaShape<T, KF>::W;
-    constexpr bool kf = KF;
+    constexpr int TJ = TmaShape<KF>::TJ, W = TmaShape<KF>::W;
     const Lev& L = ctx.lev[l];
-    // FP32 only: the FP64 pass measured slower through shared memory (104-117
-    // against 87 us at 257^3), the FP32 pass faster (49.6 against 51.2 us)
-    if (sizeof(T) != 4 || !ctx.tma_ok || L.P > 256 || op.dex[0] || L.ny < 3 || L.nz < 3) return 0;
+    if (!ctx.tma_ok || L.P > 256 || op.dex[0] || L.ny < 3 || L.nz < 3) return 0;
     ColourSplit cs;
     if (!make_split(L, W, cs)) return 0;
     const int oc = c ^ 1;
-    const T* uo = oc == 0 ? H.U[l][H.ri[l]] : H.U[l][H.bi[l]] + L.half;
+    const float* uo = oc == 0 ? H.U[l][H.ri[l]] : H.U[l][H.bi[l]] + L.half;
     CUtensorMap mU, mKo, mKc, mF;
     std::memset(&mKo, 0, sizeof(mKo));
     std::memset(&mKc, 0, sizeof(mKc));
-    if (!encode_half<T>(&mU, uo, L, TJ + 2) || !encode_half<T>(&mF, fh, L, TJ)) return 0;
-    if (kf && (!encode_half<T>(&mKo, op.k[oc], L, TJ + 2) || !encode_half<T>(&mKc, op.k[c], L, TJ))) return 0;
+    if (!encode_half(&mU, uo, L, TJ + 2) || !encode_half(&mF, fh, L, TJ)) return 0;
+    if (KF && (!encode_half(&mKo, op.k[oc], L, TJ + 2) || !encode_half(&mKc, op.k[c], L, TJ))) return 0;
     TmaColour tc;
     std::memset(&tc, 0, sizeof(tc));
-    auto pad128 = [](unsigned elems) { return (unsigned)((elems * sizeof(T) + 127) / 128 * 128 / sizeof(T)); };
+    auto pad128 = [](unsigned elems) { return (unsigned)((elems * sizeof(float) + 127) / 128 * 128 / sizeof(float)); };
     tc.tile_elems = pad128((unsigned)L.P * (TJ + 2));
     tc.own_elems = pad128((unsigned)L.P * TJ);
-    tc.slot_bytes = (unsigned)(L.P * sizeof(T)) * ((TJ + 2) * (kf ? 2 : 1) + TJ * (kf ? 2 : 1));
-    const size_t smem = kf ? tma_smem_bytes<T, true>(tc) : tma_smem_bytes<T, false>(tc);
+    tc.slot_bytes = (unsigned)(L.P * sizeof(float)) * ((TJ + 2) + TJ) * (KF ? 2 : 1);
+    const size_t smem = tma_smem_bytes<float, KF>(tc);
     if (smem > 220 * 1024) return 0;
     // tiles for the blocks that fit on an SM (shared memory, threads, at most
-    // MPS_TMA_BPS): each tile streams its planes plus two halo planes, so
+    // TmaShape::BPS): each tile streams its planes plus two halo planes, so
     // more tiles re-read more
-    const int bps = std::max(1, std::min({(int)(227 * 1024 / (smem + 1024)), 2048 / (TJ * 32), TmaShape<T, KF>::BPS}));
+    const int bps = std::max(1, std::min({(int)(227 * 1024 / (smem + 1024)), 2048 / (TJ * 32), TmaShape<KF>::BPS}));
     // the interior box of the split: rows 1 .. jhi, planes 1 .. khi (one cell
     // short of merged last cells); the shell blocks take every other row
     tc.jhi = cs.b.hi[1];
@@ -849,15 +848,15 @@ static int colour_pass_tma_kf(Ctx& ctx, Hier<T>& H, const KOp<T>& op, int l, int
         }
         return 1;
     };
-    if (L.uniform) return launch(k_colour_tma<T, W, TJ, KF, true>);
-    return launch(k_colour_tma<T, W, TJ, KF, false>);
+    if (L.uniform) return launch(k_colour_tma<float, W, TJ, KF, true>);
+    return launch(k_colour_tma<float, W, TJ, KF, false>);
 }
-template <class T>
-static int colour_pass_tma(Ctx& ctx, Hier<T>& H, const KOp<T>& op, int l, int c, T* out, const T* fh, T om)
+static int colour_pass_tma(Ctx& ctx, Hier<float>& H, const KOp<float>& op, int l, int c, float* out, const float* fh,
+                           float om)
 {
     // (a coefficient with uniform segments is not staged)
-    if (op.k[0] && !op.seg) return colour_pass_tma_kf<T, true>(ctx, H, op, l, c, out, fh, om);
-    return colour_pass_tma_kf<T, false>(ctx, H, op, l, c, out, fh, om);
+    if (op.k[0] && !op.seg) return colour_pass_tma_kf<true>(ctx, H, op, l, c, out, fh, om);
+    return colour_pass_tma_kf<false>(ctx, H, op, l, c, out, fh, om);
 }
 
 // the attributes the shared-memory colour pass needs, set outside any stream
@@ -871,7 +870,7 @@ static bool tma_prepare(int dev)
         auto set = [&](auto kern) {
             return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess;
         };
-        constexpr int W = TmaShape<float, true>::W, JK = TmaShape<float, true>::TJ, JU = TmaShape<float, false>::TJ;
+        constexpr int W = TmaShape<true>::W, JK = TmaShape<true>::TJ, JU = TmaShape<false>::TJ;
         bool ok = set(k_colour_tma<float, W, JK, true, true>) && set(k_colour_tma<float, W, JU, false, true>) &&
                   set(k_colour_tma<float, W, JK, true, false>) && set(k_colour_tma<float, W, JU, false, false>);
         if (!ok) cudaGetLastError();
@@ -988,9 +987,9 @@ static int colour_pass(Ctx& ctx, Hier<T>& H, const Op& op, int l, int c, int zer
             return 0;
         }
     }
-    if constexpr (std::is_same<Op, KOp<T>>::value) {
+    if constexpr (std::is_same<Op, KOp<float>>::value) {
         if (l <= MPS_TMA_LEVELS - 1 && zero_state == 0) {
-            const int r = colour_pass_tma<T>(ctx, H, op, l, c, out, fh, om);
+            const int r = colour_pass_tma(ctx, H, op, l, c, out, fh, om);
             if (r < 0) return MPS_ERR_CUDA;
             if (r == 1) {
                 if (l == ctx.prof.level) prof_end(ctx);
