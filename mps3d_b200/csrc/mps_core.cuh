@@ -175,8 +175,8 @@ __device__ __forceinline__ bool nbr(const Lev& L, int ax, int s, int& i, int& j,
 // arithmetic face mean k_half = (k_l + k_r)/2 (findcellcontributions,
 // discretepde.f90:646-652), Dirichlet face 2 k_c/dx^2 (:810), no convection.
 // dex = -reac + 1/dt (:1103-1106).  k or dex may be uniform (pointer null).
-// seg (when set): per row and 32 cells along x the coefficient that all of them
-// and their face neighbours share, NaN where they differ (k_kseg).
+// seg (when set): per row the coefficient that all its cells and their face
+// neighbours share, NaN where they differ (k_kseg).
 template <class T>
 struct KOp {
     const T* k[2];
@@ -184,7 +184,6 @@ struct KOp {
     const T* dex[2];
     T dexc;
     const T* seg;
-    int nseg;  // segments per row
 };
 // The words of an operator detection: largest magnitudes of the velocity, the
 // reaction, the coefficient less its first cell's, the source, the guess and the

@@ -385,10 +385,12 @@ __device__ __forceinline__ void group_rows(const Lev& L, const KOp<T>& op, int c
     row_finish<T, W, U, UNI, IN>(L, op, c, u, row, j, k, h0, q, o0, kc4, acc, wsum, byz, ax, akx, diag, off);
 }
 
-// group_rows of an interior group where the operator knows the rows' uniform
-// segments: such a group evaluates with one coefficient and reads no field, which
-// takes 2 of the pass's 5 half-fields.  A dielectric is constant outside its
-// interfaces.  Finest colour pass at 257^3 with a slab:
+// group_rows of an interior group where the operator knows the rows of one
+// coefficient: such a row evaluates with it and reads no field, which takes 2 of the
+// pass's 5 half-fields.  A dielectric is constant outside its interfaces.  By rows,
+// so that the lanes of a warp seldom differ: with 32-cell segments an interface across x
+// put both evaluations into every warp (257^3, a third of the box at 4: 24.8 ms FP64
+// against 22.2 with the field read everywhere).  Finest colour pass at 257^3 with a slab:
 // 36.1 against 47.2 us FP32 (k_colour_tma), 71.0 against 87.3 us FP64; outer
 // residual 122 against 156 us, restriction 63.5 against 77.4 us FP32.
 template <class T, int W, class U, bool UNI>
@@ -396,7 +398,7 @@ __device__ __forceinline__ void seg_rows(const Lev& L, const KOp<T>& op, int c, 
                                          int h0, int q, int o0, VecW<T, W>& diag, VecW<T, W>& off)
 {
     if (op.seg) {
-        const T ks = __ldg(op.seg + row * op.nseg + (h0 >> 4));
+        const T ks = __ldg(op.seg + row);
         if (ks == ks) {
             KOp<T> one;
             one.k[0] = one.k[1] = nullptr;
@@ -1959,33 +1961,27 @@ __global__ void k_find_bvec(Lev L, const double* __restrict__ vel, const double*
                             const double* bb, const double* bt, const double* bk, const double* bf,
                             const double* __restrict__ sterm, int flux, Split<double> b);
 
-// the uniform segments of a level's coefficient: segment s of row (j,k) covers
-// the cells 32 s .. 32 s + 31; seg = their coefficient when they, their x
-// neighbours beyond the ends and the same cells of the rows j-1, j+1, k-1, k+1 all
-// have it, else NaN (also in the rows on the y/z faces, which no interior group
-// reads).  One warp per two segments.
+// the rows of one coefficient of a level: seg = the coefficient of row (j,k)'s cells
+// when they and the cells of the rows j-1, j+1, k-1, k+1 all have it, else NaN
+// (also in the rows on the y/z faces, which no interior group reads).  One warp per row.
 template <class T>
-__global__ void __launch_bounds__(TPB) k_kseg(Lev L, CSplit<T> kf, T* __restrict__ seg, int nseg)
+__global__ void __launch_bounds__(TPB) k_kseg(Lev L, CSplit<T> kf, T* __restrict__ seg)
 {
     pdl_wait();
-    const unsigned lane = threadIdx.x & 31, nb = (unsigned)(nseg + 1) / 2;
-    const unsigned w = (blockIdx.x * TPB + threadIdx.x) >> 5;
-    const unsigned row = w / nb, b = w - row * nb;
+    const unsigned lane = threadIdx.x & 31;
+    const unsigned row = (blockIdx.x * TPB + threadIdx.x) >> 5;
     if (row >= L.rows) return;
     const int k = (int)L.divNy.div(row), j = (int)row - k * L.ny;
-    const int h = (int)(32 * b + lane);
-    const bool inner = j > 0 && j < L.ny - 1 && k > 0 && k < L.nz - 1;
-    const bool he = 2 * h < L.nx, ho = 2 * h + 1 < L.nx;
+    bool ok = j > 0 && j < L.ny - 1 && k > 0 && k < L.nz - 1;
     const int ce = (j + k) & 1;  // colour of the row's even cells
     const T* ke = kf.half(ce);
     const T* ko = kf.half(ce ^ 1);
-    const int o = h + L.P * (int)row;
-    T v = inner && he ? __ldg(ke + o) : T(0);
-    const T ref = __shfl_sync(0xffffffffu, v, (int)(lane & 16));
-    bool ok = inner;
-    if (inner && he) {
+    const T ref = __ldg(ke + L.P * (int)row);
+    for (int h = (int)lane; ok && h < L.nh; h += 32) {
         // every load is issued before the first comparison (pads are read, not used);
         // the neighbour rows' even cells have the other colour
+        const int o = h + L.P * (int)row;
+        const bool ho = 2 * h + 1 < L.nx;
         const int d[4] = {-L.P, L.P, -L.P * L.ny, L.P * L.ny};
         T e[4], f[4];
 #pragma unroll
@@ -1993,17 +1989,13 @@ __global__ void __launch_bounds__(TPB) k_kseg(Lev L, CSplit<T> kf, T* __restrict
             e[q] = __ldg(ko + o + d[q]);
             f[q] = __ldg(ke + o + d[q]);
         }
-        const T own = __ldg(ko + o);
-        const bool lo = (lane & 15) == 0 && h > 0, hi = (lane & 15) == 15 && 2 * h + 2 < L.nx;
-        const T end = lo ? __ldg(ko + o - 1) : (hi ? __ldg(ke + o + 1) : ref);
-        ok = v == ref & end == ref & (!ho | own == ref);
+        const T a = __ldg(ke + o), b = __ldg(ko + o);
+        ok = a == ref & (!ho | b == ref);
 #pragma unroll
         for (int q = 0; q < 4; q++) ok = ok & e[q] == ref & (!ho | f[q] == ref);
     }
-    const unsigned m = __ballot_sync(0xffffffffu, ok);
-    const int s = (int)(2 * b + (lane >> 4));
-    if ((lane & 15) == 0 && s < nseg)
-        seg[row * (unsigned)nseg + s] = ((m >> lane) & 0xffffu) == 0xffffu ? ref : (T)NAN;
+    ok = __all_sync(0xffffffffu, ok);
+    if (lane == 0) seg[row] = ok ? ref : (T)NAN;
 }
 
 // aggregation average (volume weighted for the geometric hierarchy) of a

@@ -253,7 +253,7 @@ struct Ctx {
     // FP64 coefficient pyramid (split cell fields)
     double* pk[MAXL] = {};
     double* pka[MAXL] = {};   // arithmetic means of the finest coefficient (levels >= 1; k_restrict_coef)
-    double* seg64[MAXL] = {};  // uniform segments of the coefficient on the large levels (k_kseg)
+    double* seg64[MAXL] = {};  // rows of one coefficient on the large levels (k_kseg)
     float* seg32[MAXL] = {};
     double* preac[MAXL] = {};
     double* pv[3][MAXL] = {};
@@ -267,7 +267,7 @@ struct Ctx {
     Hier<float> h32;
     double* x64 = nullptr;  // outer iterate (mixed / fgmres)
     double* b64 = nullptr;
-    bool kseg = false;        // this solve's operators carry the segments
+    int kseg = 0;             // this solve's operators carry the rows of one coefficient: 2 most rows are, 1 fewer
     KOp<double> kop64;      // fine-level FP64 operator for outer residuals
     ROp<double> rop64;
     double* dense = nullptr;
@@ -740,7 +740,7 @@ static RestrictSplit make_restrict_split(const Lev& F, const Lev& C, const Box& 
 // tile rows and blocks per SM of the FP32 pass.  With a staged coefficient
 // (257^3 mixed plasma solve, ms): 6 rows at 3 blocks per SM 12.72-12.75, 8 rows
 // at 2 blocks 12.79-12.81, 5 rows at 4 blocks 13.40, 7 rows at 3 blocks 13.78.
-// Without one (uniform, or uniform along most segments; 257^3 Poisson / plasma,
+// Without one (uniform, or uniform in most rows; 257^3 Poisson / plasma,
 // ms): 6 rows at 3, 4, 5 blocks - / 10.73, 5.39 / 10.37, - / 10.56; 7 rows at 4
 // blocks 5.48 / 10.86, 8 rows at 4 blocks 5.13 / 10.40
 template <bool KF>
@@ -854,8 +854,8 @@ static int colour_pass_tma_kf(Ctx& ctx, Hier<float>& H, const KOp<float>& op, in
 static int colour_pass_tma(Ctx& ctx, Hier<float>& H, const KOp<float>& op, int l, int c, float* out, const float* fh,
                            float om)
 {
-    // (a coefficient with uniform segments is not staged)
-    if (op.k[0] && !op.seg) return colour_pass_tma_kf<true>(ctx, H, op, l, c, out, fh, om);
+    // (a coefficient that is one along most rows is not staged)
+    if (op.k[0] && ctx.kseg != 2) return colour_pass_tma_kf<true>(ctx, H, op, l, c, out, fh, om);
     return colour_pass_tma_kf<false>(ctx, H, op, l, c, out, fh, om);
 }
 
@@ -1684,16 +1684,16 @@ static void alloc_hier(Ctx& ctx, Hier<T>& H, bool& ok)
     ok = ok && H.AinvT && H.Dprev && H.gj;
 }
 
-// levels whose coefficient is described by uniform segments where it can be:
+// levels whose rows of one coefficient are marked where most are:
 // those bound by bytes (a smaller level's passes are bound by latency, which the
-// segment's own load would lengthen).  257^3 plasma solve without / on the finest
+// row's own load would lengthen).  257^3 plasma solve without / on the finest
 // level / on the finest two: 11.80 / 10.79 / 10.73 ms mixed, 18.0 / 15.52 / 15.44 ms
 // FP64; the 129^3 step 5.58 / 5.51 / 5.51 ms
 constexpr long long SEG_MIN_CELLS = 1 << 19;
 static bool seg_level(const Lev& L) { return (long long)L.nx * L.ny * L.nz >= SEG_MIN_CELLS && L.nx >= 32; }
 
 // the arrays of one signature; lean: only what a solve cannot do without -- no averaged-
-// face coarse coefficients and their means, no uniform segments, no cluster (its rows
+// face coarse coefficients and their means, no rows of one coefficient, no cluster (its rows
 // are eight words a cell), the transposed rows' scratch per solve
 static bool alloc_workspace(Ctx& ctx, const Signature& sig, int need64, int need32, bool lean)
 {
@@ -1715,7 +1715,7 @@ static bool alloc_workspace(Ctx& ctx, const Signature& sig, int need64, int need
         } else {
             ctx.k32[l] = (need32 && !sig.kuni) ? (float*)ctx.ar.get(b32) : nullptr;
             const bool segs = !lean && !sig.kuni && seg_level(L);
-            const size_t ns = (size_t)L.rows * ((L.nh + 15) / 16);
+            const size_t ns = L.rows;
             ctx.seg64[l] = segs ? (double*)ctx.ar.get(sizeof(double) * ns) : nullptr;
             ctx.seg32[l] = segs ? (float*)ctx.ar.get(sizeof(float) * ns) : nullptr;
             ok = ok && (!segs || (ctx.seg64[l] && ctx.seg32[l]));
@@ -1819,7 +1819,6 @@ static void set_kop(Ctx& ctx, KOp<T>* ops, T* const* kT, T* const* dexT, double 
         const Lev& L = ctx.lev[l];
         KOp<T> op;
         op.seg = nullptr;
-        op.nseg = 0;
         if (kuni) { op.k[0] = op.k[1] = nullptr; op.kc = (T)kc; }
         else { op.k[0] = kT[l]; op.k[1] = kT[l] + L.half; op.kc = T(0); }
         if (has_reac) { op.dex[0] = dexT[l]; op.dex[1] = dexT[l] + L.half; op.dexc = T(0); }
@@ -2105,20 +2104,21 @@ static int solve_impl(Ctx& ctx, const mps_grid* g, int timederiv, double dt, con
         KOp<double> k64[MAXL];
         set_kop<double>(ctx, k64, ctx.pk, ctx.dex64, k0, dtinv, sig.kuni, sig.has_reac);
         if (need32) set_kop<float>(ctx, ctx.h32.kop, ctx.k32, ctx.dex32, k0, dtinv, sig.kuni, sig.has_reac);
-        // a coefficient that is constant along most segments: at most one change in
-        // four 32-cell chunks of the rows, and in a quarter of the sampled columns
-        // (four a row) from row to row (the passes then read one word for 32 cells;
-        // where most segments differ, that word is one more)
+        // a coefficient that changes seldom: along x at most once in four 32-cell chunks of
+        // the rows, from row to row in a quarter of the sampled columns (four a row).
+        // A row with a change along x has no single coefficient: with more than one such
+        // change in two rows the colour pass stages the field as without the marks
         const unsigned long long nchunk = (unsigned long long)L0.rows * (unsigned)((L0.nx + 31) / 32);
-        ctx.kseg = !prepare_only && !sig.kuni && ctx.seg64[0] && !in.vel && hm[6] <= nchunk / 4 && hm[7] <= (unsigned long long)L0.rows;
+        ctx.kseg = 0;
+        if (!prepare_only && !sig.kuni && ctx.seg64[0] && !in.vel && hm[6] <= nchunk / 4 &&
+            hm[7] <= (unsigned long long)L0.rows)
+            ctx.kseg = hm[6] <= L0.rows / 2 ? 2 : 1;
         if (ctx.kseg) {
             auto segments = [&](auto* k, auto* seg, auto& op, int l) -> int {
                 using TT = typename std::remove_pointer<decltype(seg)>::type;
                 const Lev& L = ctx.lev[l];
                 op.seg = seg;
-                op.nseg = (L.nh + 15) / 16;
-                const long long nw = (long long)L.rows * ((op.nseg + 1) / 2);
-                pdl_launch(k_kseg<TT>, nblk(32 * nw), TPB, 0, ctx.s, L, csplit<TT>(k, L), seg, op.nseg);
+                pdl_launch(k_kseg<TT>, nblk(32LL * L.rows), TPB, 0, ctx.s, L, csplit<TT>(k, L), seg);
                 CKL();
                 return 0;
             };
@@ -2243,7 +2243,7 @@ static int solve_impl(Ctx& ctx, const mps_grid* g, int timederiv, double dt, con
     gk.ws = ctx.ar.blocks.empty() ? nullptr : ctx.ar.blocks[0];
     gk.relaxed = ctx.relaxed;
     gk.extra_q = ctx.relaxed ? ctx.extra_q : 0;
-    gk.kseg = sig.opclass == 0 && ctx.kseg;
+    gk.kseg = sig.opclass == 0 ? ctx.kseg : 0;
     gk.prof = ctx.prof.on ? 1 + ctx.prof.level : 0;  // profiled graphs carry event-record nodes
     // graphs need the buffer parities to return after one iteration
     const bool graphs = o->use_graph && ((o->nu1 + o->nu2) % 2 == 0);
@@ -2517,7 +2517,7 @@ static int solve_impl(Ctx& ctx, const mps_grid* g, int timederiv, double dt, con
     if (ctx.prof.on) {
         prof_collect(ctx);
         ctx.prof.precision_bytes = mixed ? 4 : 8;
-        ctx.prof.coeff_field = sig.opclass == 0 ? !sig.kuni && !ctx.kseg : 7;
+        ctx.prof.coeff_field = sig.opclass == 0 ? !sig.kuni && ctx.kseg != 2 : 7;
         ctx.prof.cells = ncell;
     }
     inf.launches = (int)(ctx.launches - launches0);

@@ -290,14 +290,10 @@ __global__ void __launch_bounds__(TJ * 32) k_colour_tma(Lev L, KOp<T> op, int c,
     const bool row_ok = j <= tc.jhi;
     const T cr0 = (T)L.cr[0], cr1 = (T)L.cr[1], cr2 = (T)L.cr[2];
     bool failed = false;
-    // the coefficient of a group where the staged rows hold none (KF false): the
-    // uniform one, or the segment's (k_kseg; NaN: not uniform); the plane's first
-    // is loaded before its rows are waited for
-    auto segment = [&](int row, int g) {
-        return !KF && op.seg ? __ldg(op.seg + row * op.nseg + ((W * g) >> 4)) : op.kc;
-    };
     for (int k = k0; k <= k1; k++) {
-        const T ks0 = row_ok && tc.g_lo + lane <= tc.g_hi ? segment(j + L.ny * k, tc.g_lo + lane) : op.kc;
+        // the coefficient where the staged rows hold none (KF false): the uniform one,
+        // or the row's (k_kseg; NaN: not one), loaded before the rows are waited for
+        const T ks = !KF && op.seg && row_ok ? __ldg(op.seg + (j + L.ny * k)) : op.kc;
         bool ok = true;
         if (k == k0) ok = mbar_wait(bar + slot(k - 1), parity(k - 1), TMA_WAIT_LIMIT);
         if (k == k0) ok = ok && mbar_wait(bar + slot(k), parity(k), TMA_WAIT_LIMIT);
@@ -328,13 +324,12 @@ __global__ void __launch_bounds__(TJ * 32) k_colour_tma(Lev L, KOp<T> op, int c,
                 const int h0 = W * g;
                 VecW<T, W> diag, off;
                 const VecW<T, W> own = om != T(1) ? ldv<T, W>(urow + h0) : zerov<T, W>();
-                const T ks = g == tc.g_lo + lane ? ks0 : segment(row, g);
                 if (KF || ks == ks) {
                     KOp<T> one = op;
                     one.kc = ks;
                     tile_rows<T, W, KF>(one, U0, Uym, Uyp, Uzm, Uzp, K0, Kym, Kyp, Kzm, Kzp, Kc, h0, q, cr0, cr1, cr2,
                                         diag, off);
-                } else {  // the coefficient differs near these cells: read it
+                } else {  // the coefficient differs in or beside this row: read it
                     group_rows<T, W, CSplit<T>, true, true>(L, op, c, u, row, j, k, h0, q, (int)ro + h0, diag, off);
                 }
                 const VecW<T, W> f4 = lds<T, W>(Fr + h0);

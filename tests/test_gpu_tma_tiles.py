@@ -1,6 +1,6 @@
 """The staged colour pass (k_colour_tma) at sizes that reach it: chunks of at least
 eight planes, in both tile forms -- six rows with a staged coefficient, eight rows
-with a uniform one or uniform segments -- against the register-fed pass of a handle
+with a uniform one or one along most rows -- against the register-fed pass of a handle
 made with MPS_TMA=0.  Odd and even periodic seams, zero-gradient and Dirichlet
 faces, merged sizes, rows and planes that do not divide into the tiles, rows of
 several lane groups; V(2,2) cycles on both sides, so plain and over-relaxed passes.
@@ -41,6 +41,10 @@ def _problem(shape, bc, kind):
     elif kind == "segments":
         k[:, 1 + ny // 3:1 + ny // 3 + 9, :] = 3.0
         k[nz // 2, ny // 2, nx // 2] = 1.7
+    elif kind == "x-layer":  # no row has one coefficient: the field is staged
+        k[:, :, : nx // 3] = 3.0
+    elif kind == "x-block":  # a fifth of the planes
+        k[: nz // 5, :, : nx // 3] = 3.0
     return Problem(nx, ny, nz, (1.0, 0.8, 1.2), dcoeff=k, source=rng.uniform(-1.0, 1.0, size=g), bc=bc,
                    bcvals=[0.0, 0.4, 0.0, 0.0, -0.3, 0.0])
 
@@ -56,6 +60,8 @@ CASES = {
     "uniform-ragged": ((27, 221, 191), ["DIRC", "ZGRD"] + ZG + PER, "uniform", 8),
     "segments-odd-periodic": ((45, 205, 203), PER * 3, "segments", 8),
     "segments-mixed-faces": ((70, 198, 216), ZG + DIR + PER, "segments", 8),
+    "x-layer": ((128, 160, 150), PER + DIR + ZG, "x-layer", 6),
+    "x-block": ((130, 203, 207), PER + PER + DIR, "x-block", 8),
     "segments-long-rows": ((301, 197, 201), DIR + ["DIRC", "ZGRD"] + DIR, "segments", 8),
 }
 
