@@ -390,9 +390,9 @@ __device__ __forceinline__ void group_rows(const Lev& L, const KOp<T>& op, int c
 // pass's 5 half-fields.  A dielectric is constant outside its interfaces.  By rows,
 // so that the lanes of a warp seldom differ: with 32-cell segments an interface across x
 // put both evaluations into every warp (257^3, a third of the box at 4: 24.8 ms FP64
-// against 22.2 with the field read everywhere).  Finest colour pass at 257^3 with a slab:
-// 36.1 against 47.2 us FP32 (k_colour_tma), 71.0 against 87.3 us FP64; outer
-// residual 122 against 156 us, restriction 63.5 against 77.4 us FP32.
+// against 22.2 with the field read everywhere, now 22.9).  Finest colour pass at 257^3
+// with a slab: 34.8 against 47.2 us FP32 (k_colour_tma), 71.1 against 87.3 us FP64; outer
+// residual 123 against 156 us, restriction 62.2 against 77.4 us FP32.
 template <class T, int W, class U, bool UNI>
 __device__ __forceinline__ void seg_rows(const Lev& L, const KOp<T>& op, int c, const U& u, int row, int j, int k,
                                          int h0, int q, int o0, VecW<T, W>& diag, VecW<T, W>& off)
@@ -1963,7 +1963,8 @@ __global__ void k_find_bvec(Lev L, const double* __restrict__ vel, const double*
 
 // the rows of one coefficient of a level: seg = the coefficient of row (j,k)'s cells
 // when they and the cells of the rows j-1, j+1, k-1, k+1 all have it, else NaN
-// (also in the rows on the y/z faces, which no interior group reads).  One warp per row.
+// (also in the rows on the y/z faces, which no interior group reads).  One warp per row;
+// 46 us at 257^3 FP64 with a slab.
 template <class T>
 __global__ void __launch_bounds__(TPB) k_kseg(Lev L, CSplit<T> kf, T* __restrict__ seg)
 {

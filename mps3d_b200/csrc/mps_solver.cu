@@ -1684,7 +1684,8 @@ static void alloc_hier(Ctx& ctx, Hier<T>& H, bool& ok)
     ok = ok && H.AinvT && H.Dprev && H.gj;
 }
 
-// levels whose rows of one coefficient are marked where most are:
+// levels whose rows of one coefficient are marked where most are (figures of 32-cell
+// segments, which the rows replaced):
 // those bound by bytes (a smaller level's passes are bound by latency, which the
 // row's own load would lengthen).  257^3 plasma solve without / on the finest
 // level / on the finest two: 11.80 / 10.79 / 10.73 ms mixed, 18.0 / 15.52 / 15.44 ms
@@ -1722,7 +1723,8 @@ static bool alloc_workspace(Ctx& ctx, const Signature& sig, int need64, int need
             ctx.dex32[l] = (need32 && sig.has_reac) ? (float*)ctx.ar.get(b32) : nullptr;
         }
     }
-    // (allocating it in every solve cost 17.1 against 14.1 ms for the 65^3 gradient)
+    // (kept with the signature instead of allocated for every level of every solve; the
+    // 65^3 gradient, 14 to 24 ms from run to run, does not resolve the gain)
     const bool trows = !lean && sig.transpose;
     ctx.trows = trows ? (double*)ctx.ar.get(sizeof(double) * 7 * 2 * ctx.lev[0].half) : nullptr;
     ok = ok && (ctx.trows || !trows);
