@@ -226,6 +226,7 @@ struct Ctx {
     Arena kar;      // Krylov basis (FGMRES), keyed by (length, restart)
     long long kar_n = 0;
     int kar_m = 0;
+    int kar_dims[3] = {0, 0, 0};  // the cells whose pads its vectors hold zero
     Arena inbuf;    // host-API staging of the inputs
     struct Lane {   // one host thread of the pageable copies: a stream, two pinned buffers
         cudaStream_t s = nullptr;
@@ -1781,7 +1782,18 @@ static int setup_workspace(Ctx& ctx, const Signature& sig, int need64, int need3
 // mixed precision), w, the Hessenberg column and the dot-product partials
 static int setup_krylov(Ctx& ctx, long long n, int m)
 {
-    if (ctx.kar_n == n && ctx.kar_m == m) return 0;
+    const Lev& L0 = ctx.lev[0];
+    const int dims[3] = {L0.nx, L0.ny, L0.nz};
+    if (ctx.kar_n == n && ctx.kar_m == m) {
+        if (std::equal(dims, dims + 3, ctx.kar_dims)) return 0;
+        // another grid of the same padded length: its pads held the other's cells, and
+        // the dot products run over the pads
+        CK(cudaMemsetAsync(ctx.V, 0, sizeof(double) * n * (m + 1), ctx.s));
+        CK(cudaMemsetAsync(ctx.Z, 0, sizeof(double) * n * m, ctx.s));
+        CK(cudaMemsetAsync(ctx.w, 0, sizeof(double) * n, ctx.s));
+        std::copy(dims, dims + 3, ctx.kar_dims);
+        return 0;
+    }
     destroy_graphs(ctx);
     ctx.kar.clear();
     ctx.kar_n = 0;
@@ -1810,6 +1822,7 @@ static int setup_krylov(Ctx& ctx, long long n, int m)
     }
     ctx.kar_n = n;
     ctx.kar_m = m;
+    std::copy(dims, dims + 3, ctx.kar_dims);
     return 0;
 }
 
