@@ -56,23 +56,27 @@ constexpr int CL_SMEM_MAX = 224 * 1024;   // shared-memory bytes of a block at m
 // Cells of one colour in the largest block's share of the top level at most: beyond it
 // one launch per pass on the whole chip is faster.  Explicit rows come from L2, in FP64
 // at twice the words, and the launches for row operators (convection) read them with
-// less around it than those for a cell coefficient do, so the lines differ.  Few
+// less around it than those for a cell coefficient do, so the lines differ.  Below the
+// finest level the cluster also takes over the transfers, which FP32 rows repay.  Few
 // blocks, of a level with few planes, replace launches that were small themselves.
-// us a V-cycle with the level in the cluster / with its own launches, on a B200:
-//   uniform    FP64 36^3 (2592 cells, 16 blocks) 109 / 119, 33x65x33 (3315) 131 / 122;
-//              FP32 42^3 (3528) 85 / 90, 64x64x16 (4096, 8 blocks) 103 / 89
-//   cell FP32  36^3 87 / 91; 40x33x65 104 / 95.  FP64 33^3 (1683) 111 / 121; 100x83x61
-//              (2050 at 50x41x30) 210 / 198; 150x20x10 (3000, 5 blocks) 154 / 120
-//   convection FP32 50x41x30 (2050) 81 / 87, 36^3 86 / 81; FP64 33^3 112 / 103, 64^3
-//              (1024 at 32^3) 160 / -
-//   one block  uniform FP32 64x64x1 (2048) 80 / 59, FP64 45x50x1 (1150) 81 / 84, 100x100x2
-//              (1250 at 50x50x1) 131 / 119; three blocks 48x40x6 (1920) 84 / 97
+// us a V-cycle with the level in the cluster / with its own launches, on a B200
+// (cells of the share, blocks):
+//   uniform    FP64 36^3 (2592, 16) 109 / 119, 33x65x33 (3315, 16) 131 / 122; FP32 97^3 (48^3
+//              below: 4608, 12) 147 / 150, 64x64x16 (4096, 8) 103 / 89, 116x116x28 (3364, 7) 127 / 121
+//   cell       FP64 33^3 (1683, 16) 111 / 121, 100x83x61 (2050, 15) 210 / 198; FP32 36^3 (2592, 16)
+//              87 / 91, 40x33x65 (3300, 16) 104 / 95, 89^3 (44^3 below: 3872, 11) 155 / 160
+//   convection FP64 33^3 112 / 103; FP32 50x41x30 (2050, 15) 81 / 87, 36^3 86 / 81, 81^3 (40^3 below:
+//              3200, 16) 152 / 164
+//   few blocks uniform FP32 64x64x1 (2048, 1) 80 / 59, FP64 45x50x1 (1150, 1) 81 / 84, 100x100x2
+//              (50x50x1 below: 1250, 1) 131 / 119, 48x40x6 (1920, 3) 84 / 97, 100x30x8 (3000, 4) FP64
+//              108 / 118, FP32 82 / 77
 template <class T>
-constexpr int cl_max_share(bool rows, bool row_operator, int blocks)
+constexpr int cl_max_share(bool rows, bool row_operator, bool below, int blocks)
 {
-    const int most = sizeof(T) == 4 ? (!rows ? 3600 : row_operator ? 2200 : 2600)
-                                    : (!rows ? 3000 : row_operator ? 1100 : 1750);
-    const int few = 800 + 400 * blocks;
+    int most = 3000;
+    if (sizeof(T) == 4) most = !rows ? 4700 : below ? 3900 : row_operator ? 2200 : 3250;
+    else if (rows) most = row_operator ? 1100 : 1750;
+    const int few = sizeof(T) == 4 ? 900 + 340 * blocks : 600 + 640 * blocks;
     return most < few ? most : few;
 }
 

@@ -1324,7 +1324,8 @@ static bool cl_setup(Ctx& ctx, Hier<T>& H, const Signature& sig, bool lean)
     for (int l = 0; l < ctx.nlev; l++)
         if (odd_periodic(ctx.lev[l])) odd = l;
     for (int l = odd + 1; l < ctx.nlev - 1; l++) {
-        if (!cl_layout<T>(ctx, l, *P, smem, ax, lin) || P->share > cl_max_share<T>(rows, sig.opclass == 1, P->nc))
+        if (!cl_layout<T>(ctx, l, *P, smem, ax, lin) ||
+            P->share > cl_max_share<T>(rows, sig.opclass == 1, l > 0, P->nc))
             continue;
         H.cl_l0 = l;
         break;
